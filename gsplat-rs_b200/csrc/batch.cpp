@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "bins.cuh"
 #include "cuda_check.h"
 #include "kernels.h"
 #include "renderer.h"
@@ -91,23 +92,26 @@ std::vector<ViewGroup> plan_groups(const std::vector<ViewSpec> &views,
                                    const GroupLimits &limits) {
   std::vector<ViewGroup> groups;
   ViewGroup cur{0, 0, 0};
-  uint64_t splats = 0, tiles = 0;
+  uint64_t splats = 0, tiles = 0, bins = 0;
   const uint32_t max_views = std::min<uint32_t>(std::max(limits.max_views, 1u), kMaxViewsPerLaunch);
   for (uint32_t v = 0; v < views.size(); ++v) {
     const uint64_t n = views[v].scene->n;
-    const uint64_t t = (uint64_t)((views[v].width + tile - 1) / tile) * ((views[v].height + tile - 1) / tile);
+    const uint32_t tx = (views[v].width + tile - 1) / tile, ty = (views[v].height + tile - 1) / tile;
+    const uint64_t t = (uint64_t)tx * ty, b = (uint64_t)bins_along(tx) * bins_along(ty);
     const bool fits = cur.count < max_views && splats + n <= std::min<uint64_t>(limits.max_splats, kMaxPairs) &&
                       tiles + t <= std::min<uint64_t>(limits.max_tiles, 1u << 24) &&
+                      bins + b <= kMaxBins &&
                       cur.predicted_pairs + predicted[v] <= std::min<uint64_t>(limits.max_pairs, kMaxPairs);
     if (cur.count && !fits) {
       groups.push_back(cur);
       cur = ViewGroup{v, 0, 0};
-      splats = tiles = 0;
+      splats = tiles = bins = 0;
     }
     cur.count++;
     cur.predicted_pairs += predicted[v];
     splats += n;
     tiles += t;
+    bins += b;
   }
   if (cur.count) groups.push_back(cur);
   return groups;

@@ -79,9 +79,9 @@ struct FrameCounters {
   uint32_t drawn;
   uint32_t error;
   uint32_t overflow;
-  uint32_t pairs;  // pairs written: min(keys, capacity)
+  uint32_t pairs;  // (bin, splat) pairs written
   uint32_t raster_ticket;  // persistent raster tile queue
-  unsigned long long keys;  // pairs emitted (may exceed the capacity)
+  unsigned long long keys;  // (tile, splat) pairs they stand for (may exceed the capacity)
   uint32_t sort_tickets[16];
 };
 
@@ -93,7 +93,7 @@ struct ViewDev {
   uint32_t splat_base; // first gid of the view
   uint32_t set;        // the view set (views of one scene) the view belongs to
   uint32_t tile_base;  // first global tile id of the view
-  uint32_t pad;
+  uint32_t bin_base;   // first global bin id of the view
   unsigned long long image_base;  // first pixel of the view's image
 };
 

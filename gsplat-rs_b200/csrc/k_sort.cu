@@ -335,20 +335,16 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   }
 }
 
-// Keys per thread: 8 up to 2M keys, 16 above.
+// Keys per thread: 8 up to 2M expected keys, 16 above.
 #ifndef GSR_SORT_IPT_LARGE
 #define GSR_SORT_IPT_LARGE 16
 #endif
 constexpr int kIptLarge = GSR_SORT_IPT_LARGE;
 static_assert(kIptLarge > 8, "the large tile must hold more keys per thread than the small one");
-// Sorts sized for this many keys or more run the four-blocks-per-SM pass.
+// Sorts expected to have this many keys or more run the four-blocks-per-SM pass.
 constexpr uint32_t kHugeSort = 1u << 24;
-inline uint32_t ipt_for(uint32_t capacity) {
-  return capacity <= (1u << 21) ? 8u : (uint32_t)kIptLarge;
-}
-inline uint32_t tiles_for(uint32_t capacity) {
-  uint32_t tile = kThreads * ipt_for(capacity);
-  return (capacity + tile - 1) / tile;
+inline uint32_t ipt_for(uint32_t expected) {
+  return expected <= (1u << 21) ? 8u : (uint32_t)kIptLarge;
 }
 
 }  // namespace
@@ -407,8 +403,9 @@ uint32_t device_sm_count() {
 }
 
 void launch_sort(const SortBuffers &b, cudaStream_t stream) {
-  const uint32_t tiles = tiles_for(b.capacity);
-  const uint32_t ipt = ipt_for(b.capacity);
+  const uint32_t expected = b.expected ? b.expected : b.capacity;
+  const uint32_t ipt = ipt_for(expected);
+  const uint32_t tiles = (uint32_t)(((uint64_t)b.capacity + kThreads * ipt - 1) / (kThreads * ipt));
   uint32_t *tickets = b.work;
   uint32_t *hist = b.work + 64;
   uint32_t *status = b.work + 64 + 4 * 256;
@@ -433,7 +430,7 @@ void launch_sort(const SortBuffers &b, cudaStream_t stream) {
       pass_kernel<8, kSmall><<<g, kThreads, 0, stream>>>(b.plan, p, b.begin_bit + 8 * p, b.keys0,
                                                          b.vals0, b.keys1, b.vals1, st,
                                                          tickets + p, b.error);
-    } else if (b.capacity < kHugeSort) {
+    } else if (expected < kHugeSort) {
       const uint32_t g = std::min(grid, resident_pass_blocks<kIptLarge, kLarge>());
       pass_kernel<kIptLarge, kLarge><<<g, kThreads, 0, stream>>>(
           b.plan, p, b.begin_bit + 8 * p, b.keys0, b.vals0, b.keys1, b.vals1, st, tickets + p,

@@ -1,24 +1,27 @@
-// K2: (tile, splat) pair emission, and the tile-range build. Tile ids are
-// global over the views of a batch: views[v].tile_base + local tile.
+// K2: (bin, splat) pair emission, and the bin-range build (bins.cuh: a bin is
+// 4x4 raster tiles). Bin ids are global over the views of a batch:
+// views[v].bin_base + local bin.
 //
 // Emission walks the depth-sorted visible ids. Each block takes the next
 // kEmitThreads * kEmitIpt sorted positions from an atomic ticket. A splat
 // covers, per row of its tile rect, only the span of columns its ellipse
-// reaches (tile_span.cuh), so the block first computes every row's span: each
-// warp walks the rows of its own items 32 at a time (a lane finds its item by
-// a 5-step shuffle search over the items' inclusive row counts), keeps the
-// spans in shared memory and adds their widths to the items' pair counts.
-// The block's total then gets its global pair offset from a decoupled
+// reaches (tile_span.cuh). Its unit of work is a bin row, up to four tile
+// rows: a lane computes their spans, and with them the bin columns they reach
+// and the tile pairs they stand for. Each warp walks the units of its own
+// items 32 at a time (a lane finds its item by a 5-step shuffle search over
+// the items' inclusive unit counts) and keeps the spans in shared memory.
+// The block's pair total then gets its global offset from a decoupled
 // look-back, so pairs land in exactly the order a sequential walk would write
-// them: depth order, then rect rows, then the row's columns. Each warp then
-// walks the same row windows again and writes the window's pairs 32 at a
-// time (a lane finds its row by a second search over the rows' inclusive
-// widths), so a splat covering thousands of tiles is spread over the lanes.
-// The digit histograms the tile sort needs are accumulated while the pairs
-// are written.
+// them: depth order, then bin rows, then bin columns. Each warp then walks
+// the same unit windows again and writes the window's pairs 32 at a time (a
+// lane finds its unit by a second search over the units' inclusive widths and
+// codes the tiles from the unit's spans), so a splat covering hundreds of
+// bins is spread over the lanes. The digit histograms the bin sort needs are
+// accumulated while the pairs are written.
 
 #include <algorithm>
 
+#include "bins.cuh"
 #include "device_common.cuh"
 #include "kernels.h"
 #include "tile_span.cuh"
@@ -26,23 +29,20 @@
 namespace gsr {
 namespace {
 
-// Sorted ids per thread: 2 up to GSR_EMIT_SMALL_IDS ids (more blocks in
-// flight for a single frame), 4 above (fewer blocks, each reading the view
-// table once) (tuning knob).
-#ifndef GSR_EMIT_SMALL_IDS
-#define GSR_EMIT_SMALL_IDS (1u << 21)
-#endif
-// Row spans each warp keeps between its two walks (tuning knob); rows past
-// them are computed again in the second walk.
-#ifndef GSR_EMIT_ROW_SLOTS
-#define GSR_EMIT_ROW_SLOTS 256
-#endif
 constexpr int kEmitThreads = 256;
 constexpr int kEmitWarps = kEmitThreads / 32;
-constexpr uint32_t kRowSlots = GSR_EMIT_ROW_SLOTS;
-constexpr uint64_t kEmitSmallIds = GSR_EMIT_SMALL_IDS;
+// Sorted ids per thread: 2 below kEmitLargeIds ids, 4 from there on, where
+// blocks of 1,024 ids still fill the GPU (4 resident per SM): fewer blocks,
+// each with its barriers, look-back and view table (1.0 M ids of 64 thumbnail
+// views 81 -> 71 us, 21 M ids of a mixed batch 1,852 -> 1,457 us); a 279k-id
+// frame takes 43 us instead of 33 with 4.
+constexpr uint64_t kEmitLargeIds = 600'000;
+// Units whose spans each warp keeps between its two walks (16 bytes each);
+// units past them are computed again in the second walk.
+template <int kEmitIpt>
+constexpr uint32_t kUnitSlots = kEmitIpt == 2 ? 256 : 192;
 
-inline uint32_t emit_ipt(uint64_t ids) { return ids <= kEmitSmallIds ? 2u : 4u; }
+inline uint32_t emit_ipt(uint64_t ids) { return ids < kEmitLargeIds ? 2u : 4u; }
 
 // Index of the first lane whose inclusive end exceeds x (31 when none does),
 // by a 5-step shuffle search over the warp's ascending inclusive ends.
@@ -56,18 +56,18 @@ __device__ __forceinline__ uint32_t lane_search(uint32_t incl, uint32_t x) {
   return c;
 }
 
-// One window of a warp's row walk: rows r .. round_end-1 of the items from
+// One window of a warp's unit walk: units r .. round_end-1 of the items from
 // `it` on, one per lane. Both walks take the same windows.
-struct RowWindow {
-  uint32_t inc_w;      // inclusive row end of item it + lane (clamped to the warp's last)
-  uint32_t round_end;  // one past the window's last row
+struct UnitWindow {
+  uint32_t inc_w;      // inclusive unit end of item it + lane (clamped to the warp's last)
+  uint32_t round_end;  // one past the window's last unit
   uint32_t item;       // the lane's item (valid when r + lane < round_end)
-  uint32_t row;        // the lane's row within its item
+  uint32_t row;        // the lane's bin row within its item
 };
 
-__device__ __forceinline__ RowWindow row_window(const uint32_t *s_rinc, uint32_t ib, uint32_t il,
-                                                uint32_t it, uint32_t r, uint32_t lane) {
-  RowWindow w;
+__device__ __forceinline__ UnitWindow unit_window(const uint32_t *s_rinc, uint32_t ib, uint32_t il,
+                                                  uint32_t it, uint32_t r, uint32_t lane) {
+  UnitWindow w;
   w.inc_w = s_rinc[min(it + lane, il)];
   const uint32_t win_start = it > ib ? s_rinc[it - 1] : 0u;
   const uint32_t win_end = __shfl_sync(0xffffffffu, w.inc_w, 31);
@@ -80,48 +80,86 @@ __device__ __forceinline__ RowWindow row_window(const uint32_t *s_rinc, uint32_t
   return w;
 }
 
-// Span [c0, c1) of row `ty` of splat `id` with tile rect rc.
-__device__ __forceinline__ uint2 compute_row(const EmitBuffers &b, uint32_t id, uint2 rc,
-                                             uint32_t ty, float inv_tile) {
+// A unit's spans in shared memory, by tile row of the bin (0: none), with the
+// bin columns [x, y) they reach and their tiles.
+struct UnitSpans {
+  uint2 cols;
+  uint32_t tiles;
+};
+
+// The spans of bin row `br` of splat `id` with tile rect rc, into out[4].
+__device__ __forceinline__ UnitSpans unit_spans(const EmitBuffers &b, uint32_t id, uint2 rc,
+                                                uint32_t br, float inv_tile, uint32_t *out) {
   const Record *rec = &b.records[id];
   const float4 ra = rec->a, rb = rec->b;
-  const SpanPre pre = span_pre(ra, rb);
-  return row_span(ra.x, ra.y, pre, ty, b.tile, inv_tile, rc.x & 0xffffu, rc.y & 0xffffu);
+  const uint32_t first = max(kBinEdge * br, rc.x >> 16);
+  const uint32_t end = min(kBinEdge * br + kBinEdge, rc.y >> 16);
+  *reinterpret_cast<uint4 *>(out) = make_uint4(0u, 0u, 0u, 0u);
+  RowSpans spans(ra.x, ra.y, span_pre(ra, rb), b.tile, inv_tile, rc.x & 0xffffu,
+                 rc.y & 0xffffu, first);
+  uint32_t c0 = 0xffffu, c1 = 0, tiles = 0;
+  for (uint32_t ty = first; ty < end; ++ty) {
+    const uint2 sp = spans.next();
+    if (sp.x == sp.y) continue;
+    out[ty % kBinEdge] = sp.x | (sp.y << 16);
+    c0 = min(c0, sp.x);
+    c1 = max(c1, sp.y);
+    tiles += sp.y - sp.x;
+  }
+  return {c1 ? make_uint2(c0 / kBinEdge, (c1 + kBinEdge - 1) / kBinEdge) : make_uint2(0u, 0u),
+          tiles};
+}
+
+// The bin columns [x, y) that kept spans reach.
+__device__ __forceinline__ uint2 unit_columns(uint4 sp) {
+  const uint32_t rows[kBinEdge] = {sp.x, sp.y, sp.z, sp.w};
+  uint32_t c0 = 0xffffu, c1 = 0;
+#pragma unroll
+  for (uint32_t j = 0; j < kBinEdge; ++j) {
+    c0 = min(c0, rows[j] ? rows[j] & 0xffffu : 0xffffu);
+    c1 = max(c1, rows[j] >> 16);
+  }
+  return c1 ? make_uint2(c0 / kBinEdge, (c1 + kBinEdge - 1) / kBinEdge) : make_uint2(0u, 0u);
 }
 
 template <int kEmitIpt>
 __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EmitBuffers b) {
   constexpr int kEmitItems = kEmitThreads * kEmitIpt;
   constexpr int kWarpItems = kEmitItems / kEmitWarps;
-  __shared__ uint32_t s_rinc[kEmitItems];  // inclusive row counts within the warp's items
-  __shared__ uint32_t s_cnt[kEmitItems];   // pair counts
+  constexpr uint32_t kSlots = kUnitSlots<kEmitIpt>;
+  __shared__ uint4 s_span[kEmitWarps][kSlots];  // per warp unit: four rows' first | end << 16
+  __shared__ uint32_t s_rinc[kEmitItems];  // inclusive unit counts within the warp's items
   __shared__ uint32_t s_id[kEmitItems];
   __shared__ uint2 s_rect[kEmitItems];
   __shared__ uint16_t s_vi[kEmitItems];
-  __shared__ uint32_t s_span[kEmitWarps][kRowSlots];  // c0 | c1 << 16 per warp row
   __shared__ uint32_t s_wsum[kEmitWarps];
   __shared__ uint32_t s_hist[3][256];
   __shared__ uint32_t s_block;
   __shared__ unsigned long long s_prefix;
-  // View table columns: splat base, tile base, tiles per row.
+  // View table columns: splat base, bin base, bins per row; tile pairs of the
+  // block per view.
   extern __shared__ uint32_t s_views[];
-  uint32_t *s_vsb = s_views, *s_vtb = s_views + b.num_views, *s_vtx = s_views + 2 * b.num_views;
+  uint32_t *s_vsb = s_views, *s_vbb = s_views + b.num_views, *s_vbx = s_views + 2 * b.num_views;
+  uint32_t *s_vpairs = s_views + 3 * b.num_views;
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_block = atomicAdd(&b.counters->emit_ticket, 1u);
   for (uint32_t k = tid; k < 3 * 256; k += kEmitThreads) (&s_hist[0][0])[k] = 0;
   for (uint32_t v = tid; v < b.num_views; v += kEmitThreads) {
     s_vsb[v] = b.views[v].splat_base;
-    s_vtb[v] = b.views[v].tile_base;
-    s_vtx[v] = b.views[v].p.tiles_x;
+    s_vbb[v] = b.views[v].bin_base;
+    s_vbx[v] = bins_along(b.views[v].p.tiles_x);
+    s_vpairs[v] = 0;
   }
-  __syncthreads();
   // The sorted visible ids: this frame's, or the order reused from the last
   // sort (the plan keeps its count).
   const uint32_t V = b.depth_plan->n;
+  const uint32_t *ids = b.depth_plan->final_buffer == 0 ? b.ids0 : b.ids1;
+  const float inv_tile = __fdiv_rn(1.0f, (float)b.tile);
+  const uint32_t ib = warp * kWarpItems, il = ib + kWarpItems - 1;
+  if (tid == 0) s_block = atomicAdd(&b.counters->emit_ticket, 1u);
+  __syncthreads();
   const uint32_t block = s_block;
   const uint32_t start = block * kEmitItems;
   if (start >= V) return;
-  const uint32_t *ids = b.depth_plan->final_buffer == 0 ? b.ids0 : b.ids1;
 
   uint32_t rows[kEmitIpt];
   uint32_t local_rows = 0;
@@ -135,14 +173,13 @@ __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EmitBuffers b) {
       id = ids[j];
       r = b.rects[id];
       if ((r.y & 0xffffu) > (r.x & 0xffffu) && (r.y >> 16) > (r.x >> 16)) {
-        h = (r.y >> 16) - (r.x >> 16);
+        h = bins_along(r.y >> 16) - (r.x >> 16) / kBinEdge;
         vi = find_view(b.num_views, id, [&](uint32_t v) { return s_vsb[v]; });
       }
     }
     s_id[slot] = id;
     s_rect[slot] = r;
     s_vi[slot] = (uint16_t)vi;
-    s_cnt[slot] = 0;
     rows[k] = h;
     local_rows += h;
   }
@@ -160,39 +197,36 @@ __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EmitBuffers b) {
   }
   __syncwarp();
 
-  const uint32_t tile = b.tile;
-  const float inv_tile = __fdiv_rn(1.0f, (float)tile);
-  const uint32_t ib = warp * kWarpItems, il = ib + kWarpItems - 1;
   const uint32_t rows_total = s_rinc[il];
-  // First walk: every row's span, kept for the second walk, summed per item.
+  // First walk: every unit's spans, kept for the second walk; their pairs.
+  // Units past the slots go through the last window's.
+  uint32_t local = 0;
+  unsigned long long tiles_sum = 0;
   for (uint32_t r = 0, it = ib; r < rows_total;) {
-    const RowWindow w = row_window(s_rinc, ib, il, it, r, lane);
+    const UnitWindow w = unit_window(s_rinc, ib, il, it, r, lane);
     const uint32_t my = r + lane;
     if (my < w.round_end) {
       const uint2 rc = s_rect[w.item];
-      const uint2 sp = compute_row(b, s_id[w.item], rc, (rc.x >> 16) + w.row, inv_tile);
-      if (my < kRowSlots) s_span[warp][my] = sp.x | (sp.y << 16);
-      if (sp.y > sp.x) atomicAdd(&s_cnt[w.item], sp.y - sp.x);
+      const UnitSpans u =
+          unit_spans(b, s_id[w.item], rc, (rc.x >> 16) / kBinEdge + w.row, inv_tile,
+                     reinterpret_cast<uint32_t *>(
+                         &s_span[warp][r + 32 <= kSlots ? my : kSlots - 32 + lane]));
+      local += u.cols.y - u.cols.x;
+      tiles_sum += u.tiles;
+      if (b.num_views > 1 && u.tiles) atomicAdd(&s_vpairs[s_vi[w.item]], u.tiles);
     }
     it += __popc(__ballot_sync(0xffffffffu, w.inc_w <= w.round_end));
     r = w.round_end;
   }
-  __syncwarp();
-
-  // Block exclusive scan of the per-thread pair sums.
-  uint32_t local = 0;
-#pragma unroll
-  for (int k = 0; k < kEmitIpt; ++k) {
-    const uint32_t slot = tid * kEmitIpt + k;
-    local += s_cnt[slot];
+  local = warp_sum(local);
+  tiles_sum = warp_sum(tiles_sum);
+  if (lane == 0) {
+    s_wsum[warp] = local;
+    if (tiles_sum) {
+      atomicAdd(&b.counters->keys, tiles_sum);
+      if (b.num_views == 1) atomicAdd(&b.view_counters[0].pairs, (uint32_t)tiles_sum);
+    }
   }
-  uint32_t inc = local;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= (uint32_t)o) inc += t;
-  }
-  if (lane == 31) s_wsum[warp] = inc;
   __syncthreads();
   uint32_t before = 0, total = 0;
 #pragma unroll
@@ -209,34 +243,37 @@ __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EmitBuffers b) {
   const unsigned long long prefix = s_prefix;
   if (tid == 0 && block == (V - 1) / kEmitItems) {
     const unsigned long long all = prefix + total;
-    b.counters->keys = all;
     b.counters->pairs = (uint32_t)(all < b.capacity ? all : b.capacity);
     if (all > b.capacity) b.counters->overflow = 1u;
   }
 
-  // Second walk: the pairs of each row window, 32 per round.
+  // Second walk: the pairs of each unit window, 32 per round. A window that
+  // reaches past the slots went through the last 32 of them, so windows with
+  // units there are computed again.
+  const uint32_t kept_end = rows_total <= kSlots - 32 ? kSlots : kSlots - 32;
   unsigned long long kpos = prefix + before;  // position of the warp's next pair
   for (uint32_t r = 0, it = ib; r < rows_total;) {
-    const RowWindow w = row_window(s_rinc, ib, il, it, r, lane);
-    const uint32_t my = r + lane;
-    uint32_t c0 = 0, c1 = 0, row_tile = 0, id = 0;
-    if (my < w.round_end) {
+    const UnitWindow w = unit_window(s_rinc, ib, il, it, r, lane);
+    const bool kept = r + 32 <= kept_end;
+    const uint4 *spans = &s_span[warp][kept ? r : kSlots - 32];
+    uint32_t bin = 0, id = 0;
+    uint2 cols = make_uint2(0u, 0u);
+    __syncwarp();
+    if (r + lane < w.round_end) {
       const uint2 rc = s_rect[w.item];
-      const uint32_t ty = (rc.x >> 16) + w.row;
+      const uint32_t br = (rc.x >> 16) / kBinEdge + w.row;
       id = s_id[w.item];
-      if (my < kRowSlots) {
-        const uint32_t sp = s_span[warp][my];
-        c0 = sp & 0xffffu;
-        c1 = sp >> 16;
-      } else {
-        const uint2 sp = compute_row(b, id, rc, ty, inv_tile);
-        c0 = sp.x;
-        c1 = sp.y;
-      }
+      if (kept)
+        cols = unit_columns(spans[lane]);
+      else
+        cols = unit_spans(b, id, rc, br, inv_tile,
+                          reinterpret_cast<uint32_t *>(&s_span[warp][kSlots - 32 + lane]))
+                   .cols;
       const uint32_t vi = s_vi[w.item];
-      row_tile = s_vtb[vi] + ty * s_vtx[vi] + c0;  // global id of the span's first tile
+      bin = s_vbb[vi] + br * s_vbx[vi];  // global id of the bin row's first bin
     }
-    uint32_t winc = c1 - c0;
+    __syncwarp();
+    uint32_t winc = cols.y - cols.x;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t t = __shfl_up_sync(0xffffffffu, winc, o);
@@ -247,24 +284,28 @@ __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EmitBuffers b) {
       const uint32_t myp = q + lane;
       const uint32_t j = lane_search(winc, myp);
       const uint32_t pj = __shfl_sync(0xffffffffu, winc, j ? j - 1 : 0);
-      const uint32_t tj = __shfl_sync(0xffffffffu, row_tile, j);
+      const uint32_t cj = __shfl_sync(0xffffffffu, cols.x, j);
+      const uint32_t bj = __shfl_sync(0xffffffffu, bin, j);
       const uint32_t idj = __shfl_sync(0xffffffffu, id, j);
       const unsigned long long g = kpos + myp;
       if (myp < W && g < b.capacity) {
-        const uint32_t t = tj + myp - (j ? pj : 0u);
-        b.tile_keys[g] = t;
-        b.tile_vals[g] = idj;
+        const uint32_t bc = cj + myp - (j ? pj : 0u);
+        const uint4 sp = spans[j];
+        const uint32_t rows4[kBinEdge] = {sp.x, sp.y, sp.z, sp.w};
+        const uint32_t t = bj + bc;
+        b.pair_keys[g] = (t << kBinCodeBits) | bin_code(rows4, bc);
+        b.pair_vals[g] = idj;
         atomicAdd(&s_hist[0][t & 255u], 1u);
-        // The higher digits of a round's tiles are mostly equal: one add per
+        // The higher digits of a round's bins are mostly equal: one add per
         // distinct digit instead of up to 32 colliding ones.
         const uint32_t act = __activemask();
         const uint32_t lt = lanemask_lt();
-        if (b.tile_passes > 1) {
+        if (b.bin_passes > 1) {
           const uint32_t d1 = (t >> 8) & 255u;
           const uint32_t peers = __match_any_sync(act, d1);
           if ((peers & lt) == 0) atomicAdd(&s_hist[1][d1], __popc(peers));
         }
-        if (b.tile_passes > 2) {
+        if (b.bin_passes > 2) {
           const uint32_t d2 = (t >> 16) & 255u;
           const uint32_t peers = __match_any_sync(act, d2);
           if ((peers & lt) == 0) atomicAdd(&s_hist[2][d2], __popc(peers));
@@ -276,65 +317,93 @@ __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EmitBuffers b) {
     r = w.round_end;
   }
   __syncthreads();
-  for (uint32_t q = tid; q < b.tile_passes * 256; q += kEmitThreads) {
+  if (b.num_views > 1)
+    for (uint32_t v = tid; v < b.num_views; v += kEmitThreads)
+      if (const uint32_t n = s_vpairs[v]) atomicAdd(&b.view_counters[v].pairs, n);
+  for (uint32_t q = tid; q < b.bin_passes * 256; q += kEmitThreads) {
     const uint32_t n = (&s_hist[0][0])[q];
-    if (n) atomicAdd(&b.tile_hist[q], n);
+    if (n) atomicAdd(&b.bin_hist[q], n);
   }
 }
 
-// First position of a key >= t in the ascending keys[0, K).
-__device__ __forceinline__ uint32_t lower_bound(const uint32_t *keys, uint32_t K, uint32_t t) {
-  uint32_t lo = 0, hi = K;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (keys[mid] < t) lo = mid + 1;
-    else hi = mid;
+// Transpose of the warp's 32x32 bit matrix (lane l holds row l): lane l gets
+// bit l of every lane.
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, uint32_t lane) {
+  uint32_t low = 0x0000ffffu;
+#pragma unroll
+  for (uint32_t j = 16; j >= 1; j >>= 1) {
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+    x = (lane & j) ? ((y >> j) & low) | (x & ~low) : (x & low) | ((y << j) & ~low);
+    low ^= low << (j / 2);
   }
-  return lo;
+  return x;
 }
 
-// Tile boundaries of the sorted keys: four keys per thread (one 16-byte
-// load) plus the neighbour on each side. The first num_views threads also
-// count each view's pairs: its tiles are one contiguous id range, so its
-// pairs are one run of the sorted keys.
-__global__ void ranges_kernel(const SortPlan *__restrict__ plan, const uint32_t *k0,
-                              const uint32_t *k1, const FrameCounters *__restrict__ counters,
-                              uint2 *__restrict__ ranges, const ViewDev *__restrict__ views,
-                              uint32_t num_views, ViewCounters *__restrict__ view_counters) {
+// Bin boundaries of the sorted keys, and their codes as one word per tile of
+// the bin and 32 keys (tile_word in bins.cuh), the form a tile's raster walks.
+// A warp takes 256 keys. A lane's 16 tile bits of two keys, 32 apart, make one
+// word, and the transpose of the warp's 32 words (five exchanges) gives lane t
+// tile t's word of the first 32 keys and lane 16 + t that of the second; eight
+// words a tile are written as one 32-byte sector. One ballot per tile instead
+// took 1,100 instructions per 256 keys (113 us for 18 M pairs). The words go
+// to the key buffer the sort has left free (half a word per key). The frame
+// overflows when the tile pairs the keys stand for exceed the capacity.
+__global__ void __launch_bounds__(256) ranges_kernel(const SortPlan *__restrict__ plan,
+                                                     uint32_t *k0, uint32_t *k1,
+                                                     FrameCounters *__restrict__ counters,
+                                                     uint64_t capacity,
+                                                     uint2 *__restrict__ ranges) {
   const uint32_t K = counters->pairs;
-  const uint32_t *keys = plan->final_buffer == 0 ? k0 : k1;
-  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid < num_views) {  // the first view starts at 0, the last ends at K
-    const uint32_t first = tid ? lower_bound(keys, K, views[tid].tile_base) : 0u;
-    const uint32_t end =
-        tid + 1 < num_views ? lower_bound(keys, K, views[tid + 1].tile_base) : K;
-    view_counters[tid].pairs = end - first;
-  }
-  const uint32_t groups = (K + 3) / 4;
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < groups;
-       q += gridDim.x * blockDim.x) {
-    const uint32_t i0 = 4 * q;
-    uint32_t v[6];
-    if (i0 + 4 <= K) {
-      const uint4 x = *reinterpret_cast<const uint4 *>(keys + i0);
-      v[1] = x.x;
-      v[2] = x.y;
-      v[3] = x.z;
-      v[4] = x.w;
-    } else {
+  const bool first = plan->final_buffer == 0;
+  const uint32_t *keys = first ? k0 : k1;
+  uint32_t *words = first ? k1 : k0;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && counters->keys > capacity) counters->overflow = 1u;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t warps = gridDim.x * blockDim.x / 32, groups = (K + 255) / 256;
+  for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / 32; g < groups; g += warps) {
+    uint32_t key[kWordGroup];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) v[1 + k] = i0 + k < K ? keys[i0 + k] : 0xffffffffu;
+    for (uint32_t q = 0; q < kWordGroup; ++q) {
+      const uint32_t i = 256 * g + 32 * q + lane;
+      key[q] = i < K ? keys[i] : 0u;
     }
-    v[0] = i0 > 0 ? keys[i0 - 1] : 0xffffffffu;
-    v[5] = i0 + 4 < K ? keys[i0 + 4] : 0xffffffffu;
+    // the neighbours of the group's keys (out of the list: an id no bin has)
+    uint32_t before = ~0u, after = ~0u;
+    if (lane == 0 && g > 0) before = keys[256 * g - 1] >> kBinCodeBits;
+    if (lane == 31 && 256 * g + 256 < K) after = keys[256 * g + 256] >> kBinCodeBits;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint32_t i = i0 + k;
-      if (i >= K) break;
-      const uint32_t t = v[1 + k];
-      if (i == 0 || v[k] != t) ranges[t].x = i;
-      if (i + 1 == K || v[2 + k] != t) ranges[t].y = i + 1;
+    for (uint32_t q = 0; q < kWordGroup; ++q) {
+      const uint32_t i = 256 * g + 32 * q + lane;
+      const uint32_t bin = key[q] >> kBinCodeBits;
+      uint32_t prev = __shfl_up_sync(0xffffffffu, bin, 1);
+      uint32_t next = __shfl_down_sync(0xffffffffu, bin, 1);
+      const uint32_t last_before =
+          q > 0 ? __shfl_sync(0xffffffffu, key[q > 0 ? q - 1 : 0], 31) >> kBinCodeBits : before;
+      const uint32_t first_after =
+          q + 1 < kWordGroup
+              ? __shfl_sync(0xffffffffu, key[q + 1 < kWordGroup ? q + 1 : q], 0) >> kBinCodeBits
+              : after;
+      if (lane == 0) prev = last_before;
+      if (lane == 31) next = first_after;
+      if (i < K) {
+        if (prev != bin) ranges[bin].x = i;
+        if (i + 1 == K || next != bin) ranges[bin].y = i + 1;
+      }
     }
+    uint32_t mine[kWordGroup / 2];
+#pragma unroll
+    for (uint32_t q = 0; q < kWordGroup / 2; ++q)
+      mine[q] = transpose32(bin_code_tiles(key[2 * q]) | bin_code_tiles(key[2 * q + 1]) << 16,
+                            lane);
+    // lane t: words 0, 2, 4, 6 of tile t; lane 16 + t: words 1, 3, 5, 7
+    uint32_t other[kWordGroup / 2];
+#pragma unroll
+    for (uint32_t q = 0; q < kWordGroup / 2; ++q)
+      other[q] = __shfl_xor_sync(0xffffffffu, mine[q], 16);
+    const bool odd = lane >= 16;
+    uint4 *out = reinterpret_cast<uint4 *>(&words[tile_word(kWordGroup * g, lane & 15u)]);
+    out[odd] = odd ? make_uint4(other[2], mine[2], other[3], mine[3])
+                   : make_uint4(mine[0], other[0], mine[1], other[1]);
   }
 }
 
@@ -371,29 +440,34 @@ uint64_t emit_blocks(uint64_t ids) {
 }
 
 uint64_t emit_status_words(uint64_t capacity) {
-  return std::max(emit_blocks(std::min(capacity, kEmitSmallIds)), emit_blocks(capacity));
+  return std::max(emit_blocks(std::min(capacity, kEmitLargeIds - 1)), emit_blocks(capacity));
 }
 
 void launch_emit(const EmitBuffers &b, cudaStream_t stream) {
   const uint32_t blocks = (uint32_t)emit_blocks(b.n);
   if (blocks == 0 || b.num_views == 0) return;
-  const size_t smem = 3 * 4 * b.num_views;
+  const size_t smem = 4 * 4 * b.num_views;
+  // The static arrays and the largest view table together pass 48 KB.
+  static const bool configured = [] {
+    const int most = (int)(4 * 4 * kMaxViewsPerLaunch);
+    cudaFuncSetAttribute(emit_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    cudaFuncSetAttribute(emit_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    return true;
+  }();
+  (void)configured;
   if (emit_ipt(b.n) == 2)
     emit_kernel<2><<<blocks, kEmitThreads, smem, stream>>>(b);
   else
     emit_kernel<4><<<blocks, kEmitThreads, smem, stream>>>(b);
 }
 
-void launch_ranges(const SortPlan *tile_plan, const uint32_t *keys0, const uint32_t *keys1,
-                   const FrameCounters *counters, uint32_t capacity, uint2 *ranges,
-                   const ViewDev *views, uint32_t num_views, ViewCounters *view_counters,
+void launch_ranges(const SortPlan *bin_plan, uint32_t *keys0, uint32_t *keys1,
+                   FrameCounters *counters, uint32_t capacity, uint2 *ranges,
                    cudaStream_t stream) {
-  uint32_t blocks = (capacity + 255) / 256;
+  uint32_t blocks = (capacity + 2047) / 2048;
   const uint32_t cap = 8 * device_sm_count();
   blocks = blocks < cap ? (blocks ? blocks : 1) : cap;
-  blocks = std::max(blocks, (num_views + 255) / 256);
-  ranges_kernel<<<blocks, 256, 0, stream>>>(tile_plan, keys0, keys1, counters, ranges, views,
-                                            num_views, view_counters);
+  ranges_kernel<<<blocks, 256, 0, stream>>>(bin_plan, keys0, keys1, counters, capacity, ranges);
 }
 
 const void *run_init_kernel_entry() { return reinterpret_cast<const void *>(&run_init_kernel); }

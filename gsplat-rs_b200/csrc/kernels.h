@@ -60,6 +60,9 @@ struct SortBuffers {
   const uint32_t *hist;
   // The scratch's tickets and histograms are already zero (else one memset).
   bool scratch_zeroed = false;
+  // Items to tune the tiles for where far fewer than `capacity` are likely
+  // (0: capacity). Any count up to the capacity is sorted.
+  uint32_t expected = 0;
 };
 constexpr uint32_t kSortScratchHeadWords = 64 + 4 * 256;  // tickets and histograms
 uint64_t sort_work_words(uint32_t capacity, uint32_t passes);
@@ -67,18 +70,21 @@ uint64_t sort_work_words(uint32_t capacity, uint32_t passes);
 // plan and pass kernels on `stream`.
 void launch_sort(const SortBuffers &b, cudaStream_t stream);
 
-// ---- K2: tile-pair emission over the depth-sorted visible ids ------------
+// ---- K2: (bin, splat) pair emission over the depth-sorted visible ids -----
+// A bin is 4x4 tiles (bins.cuh); a pair's key codes the bin's tiles the splat
+// reaches. counters->keys and view_counters[].pairs count those tiles.
 struct EmitBuffers {
   const SortPlan *depth_plan;      // selects the buffer holding the sorted ids; n = their count
   const uint32_t *ids0, *ids1;     // depth-sorted gids, [visible]
   const uint2 *rects;              // [gid] tile rects
   const Record *records;           // [gid] raster records (row spans)
-  uint32_t *tile_keys, *tile_vals; // [capacity] output pairs (global tile id, gid)
+  uint32_t *pair_keys, *pair_vals; // [capacity] output pairs (global bin id and tile code, gid)
   uint64_t capacity;
   unsigned long long *status;      // [emit_blocks(n)] look-back words, zeroed
   FrameCounters *counters;
-  uint32_t *tile_hist;             // [passes][256] digit histograms of the tile ids, zeroed
-  uint32_t tile_passes;
+  ViewCounters *view_counters;     // pairs zeroed
+  uint32_t *bin_hist;              // [passes][256] digit histograms of the bin ids, zeroed
+  uint32_t bin_passes;
   uint32_t n;                      // total splats over the views (upper bound of visible)
   const ViewDev *views;
   uint32_t num_views;              // at most kMaxViewsPerLaunch
@@ -89,11 +95,12 @@ uint64_t emit_blocks(uint64_t ids);              // emission blocks (look-back w
 uint64_t emit_status_words(uint64_t capacity);   // look-back words any n <= capacity needs
 void launch_emit(const EmitBuffers &b, cudaStream_t stream);
 
-// ---- tile ranges from the tile-sorted keys -------------------------------
-// Also writes each view's pair count (view_counters[v].pairs).
-void launch_ranges(const SortPlan *tile_plan, const uint32_t *keys0, const uint32_t *keys1,
-                   const FrameCounters *counters, uint32_t capacity, uint2 *ranges,
-                   const ViewDev *views, uint32_t num_views, ViewCounters *view_counters,
+// ---- bin ranges and tile bits from the bin-sorted keys -------------------
+// The bits (one per tile of a bin and list position) replace the contents of
+// the key buffer that does not hold the sorted keys. Also flags the overflow
+// of a run whose tile pairs exceed the capacity.
+void launch_ranges(const SortPlan *bin_plan, uint32_t *keys0, uint32_t *keys1,
+                   FrameCounters *counters, uint32_t capacity, uint2 *ranges,
                    cudaStream_t stream);
 
 // ---- K4: tile raster ------------------------------------------------------
@@ -102,9 +109,9 @@ struct RasterArgs {
   const ViewDev *views;
   uint32_t num_views;
   uint32_t total_tiles;            // global tiles over the views
-  const uint2 *ranges;             // [total_tiles] list ranges
-  const SortPlan *plan;            // selects the buffer holding the sorted ids
-  const uint32_t *ids0, *ids1;
+  const uint2 *ranges;             // [bins] list ranges
+  const SortPlan *plan;            // selects the buffers of the sorted ids and the tile bits
+  const uint32_t *keys0, *ids0, *keys1, *ids1;
   const Record *records;
   uint32_t *images;
   FrameCounters *counters;         // raster_ticket is the persistent tile queue

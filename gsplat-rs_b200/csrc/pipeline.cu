@@ -6,6 +6,7 @@
 #include <cstring>
 #include <string>
 
+#include "bins.cuh"
 #include "kernels.h"
 #include "cuda_check.h"
 #include "pipeline.h"
@@ -16,6 +17,10 @@ namespace {
 inline uint64_t align256(uint64_t v) { return (v + 255) & ~uint64_t(255); }
 constexpr uint64_t kMaxSortItems = (1u << 30) - 1;
 constexpr uint64_t kInitialPairsPerSplat = 16;
+// The pair capacity counts tile pairs; a run of that many has about this many
+// times fewer (bin, splat) pairs: 3.3 at 279k splats and 1920x1080 (whose
+// capacity is 2.6 times its tile pairs), 9 at 3M and 3840x2160.
+constexpr uint64_t kPairsPerBinPair = 8;
 }  // namespace
 
 DeviceBuffer::~DeviceBuffer() { release(); }
@@ -59,9 +64,9 @@ void DeviceBuffer::reset(uint64_t bytes) {
   bytes_ = bytes;
 }
 
-uint32_t tile_sort_passes(uint32_t num_tiles) {
+uint32_t bin_sort_passes(uint32_t num_bins) {
   uint32_t bits = 0;
-  while (bits < 32 && (1ull << bits) < num_tiles) ++bits;
+  while (bits < 32 && (1ull << bits) < num_bins) ++bits;
   return std::max(1u, (bits + 7) / 8);
 }
 
@@ -120,7 +125,6 @@ Pipeline::Pipeline(int device, cudaStream_t stream) : device_(device), stream_(s
   sm_count_ = (uint32_t)sms;
   for (auto &ev : ev_) GSR_CUDA(cudaEventCreate(&ev));
   for (auto &ev : slot_ev_) GSR_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-
   GSR_CUDA(cudaMallocHost(&counters_host_, sizeof(FrameCounters)));
   std::memset(counters_host_, 0, sizeof(FrameCounters));
   // fixed scratch: [counters | key hist | tile hist] zeroed per run, then
@@ -137,9 +141,9 @@ Pipeline::Pipeline(int device, cudaStream_t stream) : device_(device), stream_(s
   GSR_CUDA(cudaMemset(fixed_.get(), 0, off));
   counters_ = fixed_.as<FrameCounters>(o_counters);
   key_hist_ = fixed_.as<uint32_t>(o_khist);
-  tile_hist_ = fixed_.as<uint32_t>(o_thist);
+  bin_hist_ = fixed_.as<uint32_t>(o_thist);
   depth_plan_ = fixed_.as<SortPlan>(o_dplan);
-  tile_plan_ = fixed_.as<SortPlan>(o_tplan);
+  bin_plan_ = fixed_.as<SortPlan>(o_tplan);
   sticky_ = fixed_.as<uint32_t>(o_sticky);
   (void)zero_end;
 }
@@ -209,7 +213,7 @@ Pipeline::Layout Pipeline::plan_views(const ViewSpec *views, uint32_t count,
   l.views = count;
   views_host_.resize(count);
   sets_host_.clear();
-  uint64_t splats = 0, blocks = 0, tiles = 0;
+  uint64_t splats = 0, blocks = 0, tiles = 0, bins = 0;
   for (uint32_t v = 0; v < count; ++v) {
     const ViewSpec &vs = views[v];
     if (!camera_valid(vs.camera)) throw Error(Code::InvalidArgument, "invalid camera");
@@ -222,6 +226,7 @@ Pipeline::Layout Pipeline::plan_views(const ViewSpec *views, uint32_t count,
     d.sc = vs.scene->dev;
     d.splat_base = (uint32_t)splats;
     d.tile_base = (uint32_t)tiles;
+    d.bin_base = (uint32_t)bins;
     d.image_base = image_bases[v];
     // Consecutive views of one scene form a view set (one scene read in K1).
     if (sets_host_.empty() || views[v - 1].scene != vs.scene ||
@@ -233,16 +238,19 @@ Pipeline::Layout Pipeline::plan_views(const ViewSpec *views, uint32_t count,
     d.set = (uint32_t)sets_host_.size() - 1;
     splats += vs.scene->n;
     tiles += d.p.num_tiles;
+    bins += (uint64_t)bins_along(d.p.tiles_x) * bins_along(d.p.tiles_y);
     l.max_planes = std::max(l.max_planes, vs.scene->dev.planes);
   }
   if (splats > kMaxSortItems)
     throw Error(Code::Unsupported, "splats over the views of one run exceed 2^30 - 1");
-  if (tiles > (1u << 24)) throw Error(Code::Unsupported, "too many tiles in one run");
+  if (tiles > (1u << 24) || bins > kMaxBins)
+    throw Error(Code::Unsupported, "too many tiles in one run");
   l.total_splats = (uint32_t)splats;
   l.sets = (uint32_t)sets_host_.size();
   l.total_blocks = (uint32_t)blocks;
   l.total_tiles = (uint32_t)tiles;
-  l.tile_passes = tile_sort_passes(l.total_tiles);
+  l.total_bins = (uint32_t)bins;
+  l.bin_passes = bin_sort_passes(l.total_bins);
   return l;
 }
 
@@ -322,13 +330,13 @@ void Pipeline::ensure_workspace(const Layout &l) {
     note_regrowth(std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() -
                                                             t_grow).count());
   }
-  if (l.total_tiles > tile_cap_ || !tile_ws_.get()) {
+  if (l.total_bins > bin_cap_ || !bin_ws_.get()) {
     const auto t_grow = std::chrono::steady_clock::now();
     GSR_CUDA(cudaStreamSynchronize(stream_));
     drop_graph();
-    tile_cap_ = std::max(l.total_tiles, tile_cap_ + tile_cap_ / 2);
-    tile_ws_.reset(align256(8ull * std::max<uint32_t>(tile_cap_, 1)), stream_);
-    ranges_ = tile_ws_.as<uint2>();
+    bin_cap_ = std::max(l.total_bins, bin_cap_ + bin_cap_ / 2);
+    bin_ws_.reset(align256(8ull * std::max<uint32_t>(bin_cap_, 1)), stream_);
+    ranges_ = bin_ws_.as<uint2>();
     note_regrowth(std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() -
                                                             t_grow).count());
   }
@@ -356,7 +364,7 @@ void Pipeline::ensure_workspace(const Layout &l) {
 }
 
 void Pipeline::ensure_key_workspace(uint64_t capacity) {
-  const uint32_t passes = 3;  // enough for any tile count below 2^24
+  const uint32_t passes = 3;  // enough for any bin count
   if (key_cap_ >= capacity && key_ws_.get()) return;
   if (capacity > kMaxSortItems)
     throw Error(Code::Unsupported, "tile pair count " + std::to_string(capacity) +
@@ -375,11 +383,11 @@ void Pipeline::ensure_key_workspace(uint64_t capacity) {
   uint64_t o_v1 = off; off += align256(4ull * cap);
   uint64_t o_work = off; off += align256(4 * words);
   key_ws_.reset(off, stream_);
-  tile_keys0_ = key_ws_.as<uint32_t>(o_k0);
-  tile_vals0_ = key_ws_.as<uint32_t>(o_v0);
-  tile_keys1_ = key_ws_.as<uint32_t>(o_k1);
-  tile_vals1_ = key_ws_.as<uint32_t>(o_v1);
-  tile_sort_work_ = key_ws_.as<uint32_t>(o_work);
+  pair_keys0_ = key_ws_.as<uint32_t>(o_k0);
+  pair_vals0_ = key_ws_.as<uint32_t>(o_v0);
+  pair_keys1_ = key_ws_.as<uint32_t>(o_k1);
+  pair_vals1_ = key_ws_.as<uint32_t>(o_v1);
+  pair_sort_work_ = key_ws_.as<uint32_t>(o_work);
   key_cap_ = cap;
   debug_pairs_.reset(0, stream_);
   note_regrowth(std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() -
@@ -393,10 +401,10 @@ RunInit Pipeline::make_run_init(const Layout &l) const {
   init.zero[1] = view_ws_.as<uint32_t>();
   init.zero_words[1] = view_zero_bytes_ / 4;
   init.zero[2] = reinterpret_cast<uint32_t *>(ranges_);
-  init.zero_words[2] = 2ull * l.total_tiles;
+  init.zero_words[2] = 2ull * l.total_bins;
   init.zero[3] = depth_sort_work_;
   init.zero_words[3] = kSortScratchHeadWords;
-  init.zero[4] = tile_sort_work_;
+  init.zero[4] = pair_sort_work_;
   init.zero_words[4] = kSortScratchHeadWords;
   if (l.views <= kRunInlineViews && !batch_mode_) {
     init.inline_views = l.views;
@@ -430,27 +438,29 @@ void Pipeline::launch_all(const Layout &l, uint32_t *images, const HostSinks &si
   record(2);
 
   EmitBuffers eb{depth_plan_, vis_vals0_,  vis_vals1_, rects_,        records_,
-                 tile_keys0_, tile_vals0_, key_cap_,   emit_status_,  counters_,
-                 tile_hist_,  l.tile_passes, l.total_splats, views_dev,  l.views,
-                 tile_};
+                 pair_keys0_, pair_vals0_, key_cap_,   emit_status_,  counters_,
+                 view_counters_, bin_hist_, l.bin_passes, l.total_splats, views_dev,
+                 l.views, tile_};
   launch_emit(eb, stream_);
   if (debug_) {
-    GSR_CUDA(cudaMemcpyAsync(debug_pairs_.as<uint32_t>(), tile_keys0_, 4 * key_cap_,
+    GSR_CUDA(cudaMemcpyAsync(debug_pairs_.as<uint32_t>(), pair_keys0_, 4 * key_cap_,
                              cudaMemcpyDeviceToDevice, stream_));
-    GSR_CUDA(cudaMemcpyAsync(debug_pairs_.as<uint32_t>(4 * key_cap_), tile_vals0_, 4 * key_cap_,
+    GSR_CUDA(cudaMemcpyAsync(debug_pairs_.as<uint32_t>(4 * key_cap_), pair_vals0_, 4 * key_cap_,
                              cudaMemcpyDeviceToDevice, stream_));
   }
   record(3);
-  SortBuffers ts{tile_keys0_, tile_vals0_, tile_keys1_, tile_vals1_, &counters_->pairs,
-                 (uint32_t)key_cap_, 0, l.tile_passes, tile_plan_, tile_sort_work_,
-                 &counters_->error, tile_hist_, true};
+  SortBuffers ts{pair_keys0_, pair_vals0_, pair_keys1_, pair_vals1_, &counters_->pairs,
+                 (uint32_t)key_cap_, kBinCodeBits, l.bin_passes, bin_plan_, pair_sort_work_,
+                 &counters_->error, bin_hist_, true};
+  ts.expected = std::max<uint32_t>((uint32_t)(key_cap_ / kPairsPerBinPair), 1);
   launch_sort(ts, stream_);
   record(4);
-  launch_ranges(tile_plan_, tile_keys0_, tile_keys1_, counters_, (uint32_t)key_cap_, ranges_,
-                views_dev, l.views, view_counters_, stream_);
+  launch_ranges(bin_plan_, pair_keys0_, pair_keys1_, counters_, (uint32_t)key_cap_, ranges_,
+                stream_);
   record(5);
-  RasterArgs ra{views_dev,  l.views,  l.total_tiles, ranges_,   tile_plan_,
-                tile_vals0_, tile_vals1_, records_,  images, counters_, sticky_};
+  RasterArgs ra{views_dev,  l.views,  l.total_tiles, ranges_,   bin_plan_,
+                pair_keys0_, pair_vals0_, pair_keys1_, pair_vals1_, records_, images, counters_,
+                sticky_};
   if (debug_) {
     GSR_CUDA(cudaMemsetAsync(debug_cov_.get(), 0xff, 8ull * std::max<uint32_t>(l.total_splats, 1),
                              stream_));
@@ -828,14 +838,14 @@ RunResult Pipeline::sync() {
 
 uint32_t Pipeline::launches_per_run() const {
   // preprocess; depth sort plan + 4 passes (histograms come from K1); emit;
-  // tile sort plan + passes (histograms from K2); ranges; raster.
-  const uint32_t tile_passes = last_layout_.tile_passes;
-  return 1 + (1 + 4) + 1 + (1 + tile_passes) + 1 + 1;
+  // bin sort plan + passes (histograms from K2); ranges; raster.
+  const uint32_t bin_passes = last_layout_.bin_passes;
+  return 1 + (1 + 4) + 1 + (1 + bin_passes) + 1 + 1;
 }
 
 SortPlan Pipeline::read_plan(int which) {
   SortPlan plan;
-  GSR_CUDA(cudaMemcpyAsync(&plan, which == 0 ? depth_plan_ : tile_plan_, sizeof(SortPlan),
+  GSR_CUDA(cudaMemcpyAsync(&plan, which == 0 ? depth_plan_ : bin_plan_, sizeof(SortPlan),
                            cudaMemcpyDeviceToHost, stream_));
   GSR_CUDA(cudaStreamSynchronize(stream_));
   return plan;
@@ -873,32 +883,81 @@ std::vector<float2> Pipeline::debug_coverage(uint32_t count) {
   return out;
 }
 
+// The (tile, splat) pairs of the frame in emission order (depth order, tile
+// rows outer), from the (bin, splat) pairs: a splat's pairs lie together, bin
+// rows outer, so its tile row r is row r % 4 of its bins of that bin row.
 void Pipeline::debug_tile_pairs(std::vector<uint32_t> &tiles, std::vector<uint32_t> &ids) {
   if (!debug_ || !debug_pairs_.get())
     throw Error(Code::InvalidArgument, "debug taps were not enabled for the last frame");
   GSR_CUDA(cudaSetDevice(device_));
-  const uint64_t k = std::min<uint64_t>(last_.keys, key_cap_);
-  tiles.resize(k);
-  ids.resize(k);
-  if (k) {
-    GSR_CUDA(cudaMemcpy(tiles.data(), debug_pairs_.get(), 4 * k, cudaMemcpyDeviceToHost));
-    GSR_CUDA(cudaMemcpy(ids.data(), debug_pairs_.as<uint32_t>(4 * key_cap_), 4 * k,
+  const uint64_t n = std::min<uint64_t>(last_sinks_.counters->pairs, key_cap_);
+  std::vector<uint32_t> keys(n), vals(n);
+  if (n) {
+    GSR_CUDA(cudaMemcpy(keys.data(), debug_pairs_.get(), 4 * n, cudaMemcpyDeviceToHost));
+    GSR_CUDA(cudaMemcpy(vals.data(), debug_pairs_.as<uint32_t>(4 * key_cap_), 4 * n,
                         cudaMemcpyDeviceToHost));
+  }
+  tiles.clear();
+  ids.clear();
+  tiles.reserve(last_.keys);
+  ids.reserve(last_.keys);
+  const uint32_t tiles_x = views_host_[0].p.tiles_x, bins_x = bins_along(tiles_x);
+  for (uint64_t i = 0; i < n;) {
+    const uint32_t row = (keys[i] >> kBinCodeBits) / bins_x;
+    uint64_t end = i;
+    while (end < n && vals[end] == vals[i] && (keys[end] >> kBinCodeBits) / bins_x == row) ++end;
+    for (uint32_t r = 0; r < kBinEdge; ++r)
+      for (uint64_t k = i; k < end; ++k) {
+        const uint32_t col = (keys[k] >> kBinCodeBits) % bins_x;
+        for (uint32_t c = 0; c < kBinEdge; ++c)
+          if (bin_code_tiles(keys[k]) >> (kBinEdge * r + c) & 1u) {
+            tiles.push_back((row * kBinEdge + r) * tiles_x + col * kBinEdge + c);
+            ids.push_back(vals[k]);
+          }
+      }
+    i = end;
   }
 }
 
+// Every tile's list, as the raster takes it from its bin's.
 void Pipeline::debug_tile_ranges(uint32_t num_tiles, std::vector<uint32_t> &ranges,
                                  std::vector<uint32_t> &ids) {
   GSR_CUDA(cudaSetDevice(device_));
   SortPlan plan = read_plan(1);
-  ranges.resize(2ull * num_tiles);
-  if (num_tiles)
-    GSR_CUDA(cudaMemcpy(ranges.data(), ranges_, 4 * ranges.size(), cudaMemcpyDeviceToHost));
-  const uint64_t k = std::min<uint64_t>(last_.keys, key_cap_);
-  ids.resize(k);
-  if (k)
-    GSR_CUDA(cudaMemcpy(ids.data(), plan.final_buffer == 0 ? tile_vals0_ : tile_vals1_, 4 * k,
+  const uint64_t n = std::min<uint64_t>(last_sinks_.counters->pairs, key_cap_);
+  std::vector<uint32_t> keys(n), vals(n);
+  if (n) {
+    const bool first = plan.final_buffer == 0;
+    GSR_CUDA(cudaMemcpy(keys.data(), first ? pair_keys0_ : pair_keys1_, 4 * n,
                         cudaMemcpyDeviceToHost));
+    GSR_CUDA(cudaMemcpy(vals.data(), first ? pair_vals0_ : pair_vals1_, 4 * n,
+                        cudaMemcpyDeviceToHost));
+  }
+  const uint32_t tiles_x = views_host_[0].p.tiles_x, bins_x = bins_along(tiles_x);
+  std::vector<uint32_t> count(num_tiles, 0);
+  auto each = [&](auto f) {
+    for (uint64_t k = 0; k < n; ++k) {
+      const uint32_t bin = keys[k] >> kBinCodeBits;
+      for (uint32_t r = 0; r < kBinEdge; ++r)
+        for (uint32_t c = 0; c < kBinEdge; ++c)
+          if (bin_code_tiles(keys[k]) >> (kBinEdge * r + c) & 1u)
+            f((bin / bins_x * kBinEdge + r) * tiles_x + bin % bins_x * kBinEdge + c, vals[k]);
+    }
+  };
+  each([&](uint32_t t, uint32_t) { ++count[t]; });
+  ranges.assign(2ull * num_tiles, 0);
+  uint32_t at = 0;
+  for (uint32_t t = 0; t < num_tiles; ++t) {
+    if (count[t]) {
+      ranges[2ull * t] = at;
+      ranges[2ull * t + 1] = at + count[t];
+    }
+    const uint32_t c = count[t];
+    count[t] = at;
+    at += c;
+  }
+  ids.resize(at);
+  each([&](uint32_t t, uint32_t gid) { ids[count[t]++] = gid; });
 }
 
 }  // namespace gsr

@@ -185,12 +185,14 @@ class Pipeline {
 
  private:
   struct Layout {
-    uint32_t views = 0, total_splats = 0, total_blocks = 0, total_tiles = 0, max_planes = 1;
-    uint32_t tile_passes = 1, sets = 0;
+    uint32_t views = 0, total_splats = 0, total_blocks = 0, total_tiles = 0, total_bins = 0,
+             max_planes = 1;
+    uint32_t bin_passes = 1, sets = 0;
     bool operator==(const Layout &o) const {
       return views == o.views && sets == o.sets && total_splats == o.total_splats &&
              total_blocks == o.total_blocks && total_tiles == o.total_tiles &&
-             max_planes == o.max_planes && tile_passes == o.tile_passes;
+             total_bins == o.total_bins &&
+             max_planes == o.max_planes && bin_passes == o.bin_passes;
     }
   };
   Layout plan_views(const ViewSpec *views, uint32_t count, const uint64_t *image_bases);
@@ -257,8 +259,8 @@ class Pipeline {
   // region first (one memset per run).
   DeviceBuffer fixed_;
   FrameCounters *counters_ = nullptr;
-  uint32_t *key_hist_ = nullptr, *tile_hist_ = nullptr, *sticky_ = nullptr;
-  SortPlan *depth_plan_ = nullptr, *tile_plan_ = nullptr;
+  uint32_t *key_hist_ = nullptr, *bin_hist_ = nullptr, *sticky_ = nullptr;
+  SortPlan *depth_plan_ = nullptr, *bin_plan_ = nullptr;
   FrameCounters *counters_host_ = nullptr;  // pinned
   // Per-layout scratch.
   DeviceBuffer view_ws_;  // view table + view counters + look-back words (zeroed part)
@@ -267,19 +269,19 @@ class Pipeline {
   ViewSetDev *sets_dev_ = nullptr;
   ViewCounters *view_counters_ = nullptr;
   unsigned long long *k1_status_ = nullptr, *emit_status_ = nullptr;
-  uint32_t view_cap_ = 0, splat_cap_ = 0, tile_cap_ = 0;
+  uint32_t view_cap_ = 0, splat_cap_ = 0, bin_cap_ = 0;
   DeviceBuffer splat_ws_;
   uint32_t *vis_keys0_ = nullptr, *vis_vals0_ = nullptr, *vis_keys1_ = nullptr,
            *vis_vals1_ = nullptr, *depth_sort_work_ = nullptr;
   uint2 *rects_ = nullptr;
   Record *records_ = nullptr;
   DeviceBuffer projected_;
-  DeviceBuffer tile_ws_;
+  DeviceBuffer bin_ws_;
   uint2 *ranges_ = nullptr;
   DeviceBuffer key_ws_;
   uint64_t key_cap_ = 0;
-  uint32_t *tile_keys0_ = nullptr, *tile_vals0_ = nullptr, *tile_keys1_ = nullptr,
-           *tile_vals1_ = nullptr, *tile_sort_work_ = nullptr;
+  uint32_t *pair_keys0_ = nullptr, *pair_vals0_ = nullptr, *pair_keys1_ = nullptr,
+           *pair_vals1_ = nullptr, *pair_sort_work_ = nullptr;
   DeviceBuffer debug_pairs_;
   DeviceBuffer debug_cov_;
   ViewCounters *view_counters_pinned_ = nullptr;
@@ -358,6 +360,6 @@ class Pipeline {
   uint64_t graph_clock_ = 0;
 };
 
-uint32_t tile_sort_passes(uint32_t num_tiles);
+uint32_t bin_sort_passes(uint32_t num_tiles);
 
 }  // namespace gsr

@@ -54,11 +54,10 @@ __device__ __forceinline__ void boundary_x(const SpanPre &p, float y, float &xl,
   xr = __fmul_rn(__fadd_rn(by, r), p.inv_qa);
 }
 
-// Band [lo, hi] of tile row ty, clamped to the ellipse's y-extent.
-__device__ __forceinline__ void row_band(float cy, const SpanPre &p, uint32_t ty, uint32_t tile,
-                                         float &lo, float &hi) {
-  lo = fmaxf(__fsub_rn(__fsub_rn((float)(ty * tile), 0.5f), cy), -p.hy);
-  hi = fminf(__fsub_rn(__fsub_rn((float)(ty * tile + tile), 0.5f), cy), p.hy);
+// Pixel row (relative to the centre) above tile row ty: the band of row ty is
+// [band_edge(ty), band_edge(ty + 1)] clamped to the ellipse's y-extent.
+__device__ __forceinline__ float band_edge(float cy, uint32_t ty, uint32_t tile) {
+  return __fsub_rn(__fsub_rn((float)(ty * tile), 0.5f), cy);
 }
 
 // Columns of a non-empty band from the x-extents at its two boundaries.
@@ -78,19 +77,40 @@ __device__ __forceinline__ uint2 band_columns(float cx, const SpanPre &p, float 
   return make_uint2((uint32_t)f0, (uint32_t)f1);
 }
 
-// Columns [c0, c1) of tile row ty (c0 == c1: none); inv_tile = 1 / tile
-// exactly (tile is 8 or 16).
-__device__ __forceinline__ uint2 row_span(float cx, float cy, const SpanPre &p, uint32_t ty,
-                                          uint32_t tile, float inv_tile, uint32_t x0,
-                                          uint32_t x1) {
-  if (p.degenerate) return make_uint2(x0, x1);
-  float lo, hi;
-  row_band(cy, p, ty, tile, lo, hi);
-  if (!(lo <= hi)) return make_uint2(x0, x0);
-  float xl_lo, xr_lo, xl_hi, xr_hi;
-  boundary_x(p, lo, xl_lo, xr_lo);
-  boundary_x(p, hi, xl_hi, xr_hi);
-  return band_columns(cx, p, lo, hi, xl_lo, xr_lo, xl_hi, xr_hi, inv_tile, x0, x1);
-}
+// The column spans [x, y) (x == y: none) of consecutive tile rows from `ty`
+// on, inside the rect columns [x0, x1); inv_tile = 1 / tile exactly (tile is
+// 8 or 16). Consecutive rows share the edge between them: a non-empty row's
+// band ends are the edges clamped to [-hy, hy], so one boundary_x per edge
+// serves the row above and the row below.
+struct RowSpans {
+  float cx, cy;
+  SpanPre p;
+  uint32_t tile;
+  float inv_tile;
+  uint32_t x0, x1, ty;
+  float edge, xl, xr;  // the edge above row ty, and the ellipse's x there
+
+  __device__ __forceinline__ RowSpans(float cx_, float cy_, const SpanPre &p_, uint32_t tile_,
+                                      float inv_tile_, uint32_t x0_, uint32_t x1_, uint32_t ty_)
+      : cx(cx_), cy(cy_), p(p_), tile(tile_), inv_tile(inv_tile_), x0(x0_), x1(x1_), ty(ty_) {
+    edge = band_edge(cy, ty, tile);
+    boundary_x(p, fminf(fmaxf(edge, -p.hy), p.hy), xl, xr);
+  }
+
+  __device__ __forceinline__ uint2 next() {
+    ++ty;
+    if (p.degenerate) return make_uint2(x0, x1);
+    const float below = band_edge(cy, ty, tile);
+    const float lo = fmaxf(edge, -p.hy), hi = fminf(below, p.hy);
+    float xl_hi, xr_hi;
+    boundary_x(p, fmaxf(hi, -p.hy), xl_hi, xr_hi);
+    const uint2 sp = lo <= hi ? band_columns(cx, p, lo, hi, xl, xr, xl_hi, xr_hi, inv_tile, x0, x1)
+                              : make_uint2(x0, x0);
+    edge = below;
+    xl = xl_hi;
+    xr = xr_hi;
+    return sp;
+  }
+};
 
 }  // namespace gsr
