@@ -123,7 +123,7 @@ struct SortPlan {
   uint32_t pad;
   uint32_t skip[8];
   uint32_t src[8];
-  uint32_t digit_offset[8][256];
+  uint32_t digit_offset[4 * 256];  // [passes][256], or one wide pass's
 };
 
 }  // namespace gsr

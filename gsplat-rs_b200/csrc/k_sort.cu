@@ -95,16 +95,19 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *s
 }
 
 // Block 0 plans the passes; every block zeroes the look-back status words
-// of the tiles the actual item count needs (not the capacity's).
+// of the tiles the actual item count needs (not the capacity's). A pass has
+// 256 digits, or 256 kDpt of them (one pass: kDpt consecutive ones a thread).
+template <int kDpt>
 __global__ void __launch_bounds__(kThreads) plan_kernel(const uint32_t *__restrict__ count,
                                                         const uint32_t *__restrict__ hist,
                                                         uint32_t passes, SortPlan *plan,
                                                         uint32_t *status, uint32_t tile_stride,
                                                         uint32_t tile_items) {
+  constexpr uint32_t kDigits = kThreads * kDpt;
   const uint32_t n = *count;
-  const uint64_t used = (uint64_t)((n + tile_items - 1) / tile_items) * 256u;  // words per pass
+  const uint64_t used = (uint64_t)((n + tile_items - 1) / tile_items) * kDigits;  // words per pass
   for (uint32_t p = 0; p < passes; ++p) {
-    uint4 *dst = reinterpret_cast<uint4 *>(status + (size_t)p * tile_stride * 256u);
+    uint4 *dst = reinterpret_cast<uint4 *>(status + (size_t)p * tile_stride * kDigits);
     for (uint64_t k = blockIdx.x * (uint64_t)kThreads + threadIdx.x; k < used / 4;
          k += (uint64_t)gridDim.x * kThreads)
       dst[k] = make_uint4(0u, 0u, 0u, 0u);
@@ -116,11 +119,20 @@ __global__ void __launch_bounds__(kThreads) plan_kernel(const uint32_t *__restri
   if (d < 4) s_trivial[d] = 0;
   __syncthreads();
   for (uint32_t p = 0; p < passes; ++p) {
-    uint32_t c = hist[p * 256 + d];
+    uint32_t c[kDpt], sum = 0;
+#pragma unroll
+    for (int k = 0; k < kDpt; ++k) {
+      c[k] = hist[p * kDigits + d * kDpt + k];
+      sum += c[k];
+    }
     uint32_t total;
-    uint32_t ex = block_exclusive_scan(c, s_wsum, total);
-    plan->digit_offset[p][d] = ex;
-    if (c == n) s_trivial[p] = 1;  // n == 0 marks every pass trivial
+    uint32_t ex = block_exclusive_scan(sum, s_wsum, total);
+#pragma unroll
+    for (int k = 0; k < kDpt; ++k) {
+      plan->digit_offset[p * kDigits + d * kDpt + k] = ex;
+      ex += c[k];
+      if (c[k] == n) s_trivial[p] = 1;  // n == 0 marks every pass trivial
+    }
   }
   __syncthreads();
   if (d == 0) {
@@ -276,7 +288,7 @@ __device__ __forceinline__ void pass_tile(const SortPlan *__restrict__ plan, uin
     }
     st_relaxed_u32(&my_status[d], kFlagP | (exclusive + block_count));
   }
-  s_global[d] = plan->digit_offset[pass][d] + exclusive;
+  s_global[d] = plan->digit_offset[pass * 256 + d] + exclusive;
   __syncthreads();
 
   // Reorder the tile by digit in shared memory (small tiles).
@@ -335,6 +347,223 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   }
 }
 
+// ---- one wide pass ---------------------------------------------------------
+// A sort of 9 or 10 key bits (a bin sort of 257 to 1,024 bins) as one pass of
+// 512 or 1,024 digits, kDpt = 2 or 4 consecutive ones a thread, in place of two
+// passes of 256: 510 bins, 514k pairs 32.8 -> 24.6 us, 1,024 bins, 1.1 M pairs
+// 39.4 -> 36.9. Wider than that, or for sorts of more bits, 8-bit passes win: a
+// pass over 1.0 M keys takes 18 us with 256 digits, 22 with 512 and 30 with
+// 1,024, and 20.6 M pairs in 2,040 bins 334 us in one pass of 11 bits against
+// 297 in two. The 256-digit pass stays a kernel of its own: as this one's
+// kDpt = 1 form it ran 5% slower.
+constexpr int kWideIpt = 8;
+
+template <int kBits>
+struct WideSmem {
+  static constexpr uint32_t kTile = kThreads * kWideIpt;
+  static constexpr uint32_t kDigits = 1u << kBits;
+  // counts of a warp's digits (at most 32 kWideIpt), then their starts in the tile
+  alignas(16) uint16_t warp_hist[kWarps][kDigits];
+  uint32_t keys[kTile];
+  uint32_t vals[kTile];
+  uint32_t block_start[kDigits];
+  uint32_t global[kDigits];
+  uint32_t wsum[kWarps];
+  uint32_t tile;
+};
+
+// kN consecutive status words (kN = 2 or 4), each on its own a value
+// and its flag.
+template <int kN>
+__device__ __forceinline__ void ld_status(const uint32_t *p, uint32_t (&w)[kN]) {
+  if constexpr (kN == 2) {
+    asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];"
+                 : "=r"(w[0]), "=r"(w[1]) : "l"(p) : "memory");
+  } else {
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "l"(p) : "memory");
+  }
+}
+template <int kN>
+__device__ __forceinline__ void st_status(uint32_t *p, const uint32_t (&w)[kN]) {
+  if constexpr (kN == 2) {
+    asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(w[0]), "r"(w[1])
+                 : "memory");
+  } else {
+    asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(w[0]),
+                 "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+  }
+}
+
+// The counts of a thread's digits over every tile before `tile`: back over the
+// predecessors, kLookback (or two) rows of status words per step, adding
+// aggregates until the digits' nearest inclusive prefixes; a step restarts
+// where a word it needs is not published yet. Waits are bounded: on expiry
+// the error bit is set and the sums are incomplete.
+template <int kDpt>
+__device__ __forceinline__ void look_back(const uint32_t *status, uint32_t digits, uint32_t tile,
+                                          uint32_t d0, uint32_t (&exclusive)[kDpt],
+                                          uint32_t *error) {
+  constexpr int kBack = kDpt <= 2 ? kLookback : 2;
+#pragma unroll
+  for (int k = 0; k < kDpt; ++k) exclusive[k] = 0;
+  int32_t t = (int32_t)tile - 1;
+  uint32_t spins = 0, open = (1u << kDpt) - 1u;  // digits whose prefix was not met
+  while (t >= 0 && open) {
+    uint32_t w[kBack][kDpt];
+#pragma unroll
+    for (int q = 0; q < kBack; ++q) {
+      if (t - q >= 0) {
+        ld_status(&status[(size_t)(t - q) * digits + d0], w[q]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < kDpt; ++k) w[q][k] = kFlagP;
+      }
+    }
+    bool stalled = false;
+    int used = 0;
+#pragma unroll
+    for (int q = 0; q < kBack; ++q) {
+      if (stalled || !open) continue;
+#pragma unroll
+      for (int k = 0; k < kDpt; ++k)
+        stalled = stalled || (((open >> k) & 1u) && (w[q][k] & ~kMask) == 0);
+      if (stalled) continue;
+      ++used;
+#pragma unroll
+      for (int k = 0; k < kDpt; ++k) {
+        if (!((open >> k) & 1u)) continue;
+        exclusive[k] += w[q][k] & kMask;
+        if ((w[q][k] & ~kMask) == kFlagP) open &= ~(1u << k);
+      }
+    }
+    t -= used;
+    if (stalled) {
+      if (++spins > kSpinLimit) {
+        atomicOr(error, kErrLookbackTimeout);
+        break;
+      }
+      __nanosleep(20);
+    }
+  }
+}
+
+// A tile of the wide pass, as pass_tile: rank, publish, look back, reorder,
+// scatter.
+template <int kBits>
+__device__ __forceinline__ void wide_tile(const SortPlan *__restrict__ plan, uint32_t shift,
+                                          uint32_t n, uint32_t tile,
+                                          const uint32_t *__restrict__ in_k,
+                                          const uint32_t *__restrict__ in_v,
+                                          uint32_t *__restrict__ out_k,
+                                          uint32_t *__restrict__ out_v, uint32_t *status,
+                                          uint32_t *error, WideSmem<kBits> &sm) {
+  constexpr uint32_t kDigits = WideSmem<kBits>::kDigits, kTile = WideSmem<kBits>::kTile;
+  constexpr int kDpt = kDigits / kThreads;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t warp_base = tile * kTile + warp * 32 * kWideIpt;
+  uint32_t key[kWideIpt], val[kWideIpt], rank[kWideIpt];
+#pragma unroll
+  for (int i = 0; i < kWideIpt; ++i) {
+    const uint32_t idx = warp_base + i * 32 + lane;
+    key[i] = idx < n ? in_k[idx] : 0xffffffffu;  // ranks after every real key of the last digit
+    val[i] = idx < n ? in_v[idx] : 0u;
+  }
+  uint16_t *wh = sm.warp_hist[warp];
+  const uint32_t lt = lanemask_lt();
+#pragma unroll
+  for (int i = 0; i < kWideIpt; ++i) {
+    const uint32_t d = (key[i] >> shift) & (kDigits - 1u);
+    uint32_t peers = 0xffffffffu;
+#pragma unroll
+    for (int bit = 0; bit < kBits; ++bit) {
+      const bool set = (d >> bit) & 1u;
+      const uint32_t bal = __ballot_sync(0xffffffffu, set);
+      peers &= set ? bal : ~bal;
+    }
+    const uint32_t before = wh[d];
+    rank[i] = before + __popc(peers & lt);
+    __syncwarp();
+    if (lane == (uint32_t)(__ffs(peers) - 1)) wh[d] = (uint16_t)(before + __popc(peers));
+    __syncwarp();
+  }
+  __syncthreads();
+
+  const uint32_t d0 = threadIdx.x * kDpt;
+  uint32_t count[kDpt], word[kDpt], sum = 0;
+#pragma unroll
+  for (int k = 0; k < kDpt; ++k) {
+    count[k] = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const uint32_t c = sm.warp_hist[w][d0 + k];
+      sm.warp_hist[w][d0 + k] = (uint16_t)count[k];
+      count[k] += c;
+    }
+    word[k] = (tile == 0 ? kFlagP : kFlagA) | count[k];
+    sum += count[k];
+  }
+  uint32_t *my_status = &status[(size_t)tile * kDigits + d0];
+  st_status(my_status, word);
+  uint32_t total;
+  uint32_t run = block_exclusive_scan(sum, sm.wsum, total);
+#pragma unroll
+  for (int k = 0; k < kDpt; ++k) {
+    sm.block_start[d0 + k] = run;
+    run += count[k];
+  }
+  uint32_t exclusive[kDpt];
+  look_back<kDpt>(status, kDigits, tile, d0, exclusive, error);
+  if (tile > 0) {
+#pragma unroll
+    for (int k = 0; k < kDpt; ++k) word[k] = kFlagP | (exclusive[k] + count[k]);
+    st_status(my_status, word);
+  }
+#pragma unroll
+  for (int k = 0; k < kDpt; ++k)
+    sm.global[d0 + k] = plan->digit_offset[d0 + k] + exclusive[k];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kWideIpt; ++i) {
+    const uint32_t dg = (key[i] >> shift) & (kDigits - 1u);
+    const uint32_t pos = sm.block_start[dg] + sm.warp_hist[warp][dg] + rank[i];
+    sm.keys[pos] = key[i];
+    sm.vals[pos] = val[i];
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (uint32_t s = threadIdx.x; s < kTile; s += kThreads) {
+    const uint32_t k = sm.keys[s];
+    const uint32_t dg = (k >> shift) & (kDigits - 1u);
+    const uint32_t g = sm.global[dg] + (s - sm.block_start[dg]);
+    if (g < n) {
+      out_k[g] = k;
+      out_v[g] = sm.vals[s];
+    }
+  }
+}
+
+template <int kBits>
+__global__ void __launch_bounds__(kThreads, 3)
+    wide_kernel(const SortPlan *__restrict__ plan, uint32_t shift, const uint32_t *k0,
+                const uint32_t *v0, uint32_t *k1, uint32_t *v1, uint32_t *status,
+                uint32_t *ticket, uint32_t *error) {
+  __shared__ WideSmem<kBits> sm;
+  if (plan->skip[0]) return;
+  const uint32_t n = plan->n;
+  for (;;) {
+    if (threadIdx.x == 0) sm.tile = atomicAdd(ticket, 1u);
+    uint4 *zero = reinterpret_cast<uint4 *>(&sm.warp_hist[0][0]);
+    for (uint32_t k = threadIdx.x; k < sizeof(sm.warp_hist) / 16; k += kThreads)
+      zero[k] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    const uint32_t tile = sm.tile;
+    if ((uint64_t)tile * WideSmem<kBits>::kTile >= n) break;
+    wide_tile<kBits>(plan, shift, n, tile, k0, v0, k1, v1, status, error, sm);
+    __syncthreads();  // shared memory is reused by the next tile
+  }
+}
+
 // Keys per thread: 8 up to 2M expected keys, 16 above.
 #ifndef GSR_SORT_IPT_LARGE
 #define GSR_SORT_IPT_LARGE 16
@@ -349,7 +578,8 @@ inline uint32_t ipt_for(uint32_t expected) {
 
 }  // namespace
 
-// Scratch layout: [tickets: 64 words][hist: 4*256][status: passes*tiles*256].
+// Scratch layout: [tickets: 64 words][hist: 4*256][status: passes*tiles*256, or
+// tiles*512 or *1024 of a wide pass].
 // A workspace sized for `capacity` serves every sort of up to `capacity`
 // items: smaller sorts may run 8 items per thread where a larger one runs 16,
 // and so use more tiles, so the bound takes the 8-per-thread tile count.
@@ -370,15 +600,14 @@ int current_device() {
 }
 // Resident pass blocks on the current device (the persistent grid), looked
 // up once per device.
-template <int kIpt, int kMinBlocks>
-uint32_t resident_pass_blocks() {
+template <auto kKernel>
+uint32_t resident_blocks() {
   static std::atomic<uint32_t> cache[kMaxDevices];
   const int dev = current_device();
   uint32_t blocks = cache[dev].load(std::memory_order_relaxed);
   if (blocks == 0) {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_kernel<kIpt, kMinBlocks>,
-                                                  kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kKernel, kThreads, 0);
     blocks = device_sm_count() * (uint32_t)std::max(per_sm, 1);
     cache[dev].store(blocks, std::memory_order_relaxed);
   }
@@ -402,7 +631,25 @@ uint32_t device_sm_count() {
   return sms;
 }
 
+namespace {
+// The one pass of a wide sort; the histograms are given.
+template <int kBits>
+void launch_wide(const SortBuffers &b, cudaStream_t stream) {
+  constexpr uint32_t kTile = kThreads * kWideIpt;
+  const uint32_t tiles = std::max<uint32_t>((uint32_t)(((uint64_t)b.capacity + kTile - 1) / kTile), 1);
+  uint32_t *status = b.work + kSortScratchHeadWords;
+  plan_kernel<(1 << kBits) / kThreads>
+      <<<std::min<uint32_t>(tiles, 2 * device_sm_count()), kThreads, 0, stream>>>(
+          b.count, b.hist, 1, b.plan, status, tiles, kTile);
+  const uint32_t grid = std::min(tiles, resident_blocks<wide_kernel<kBits>>());
+  wide_kernel<kBits><<<grid, kThreads, 0, stream>>>(b.plan, b.begin_bit, b.keys0, b.vals0,
+                                                    b.keys1, b.vals1, status, b.work, b.error);
+}
+}  // namespace
+
 void launch_sort(const SortBuffers &b, cudaStream_t stream) {
+  if (b.wide_bits == 9) return launch_wide<9>(b, stream);
+  if (b.wide_bits == 10) return launch_wide<10>(b, stream);
   const uint32_t expected = b.expected ? b.expected : b.capacity;
   const uint32_t ipt = ipt_for(expected);
   const uint32_t tiles = (uint32_t)(((uint64_t)b.capacity + kThreads * ipt - 1) / (kThreads * ipt));
@@ -420,23 +667,23 @@ void launch_sort(const SortBuffers &b, cudaStream_t stream) {
           <<<grid, kThreads, 0, stream>>>(b.keys0, b.count, b.begin_bit, b.passes, hist);
   }
   const uint32_t zero_blocks = std::min<uint32_t>(grid, 2 * device_sm_count());
-  plan_kernel<<<zero_blocks, kThreads, 0, stream>>>(b.count, b.hist ? b.hist : hist, b.passes,
+  plan_kernel<1><<<zero_blocks, kThreads, 0, stream>>>(b.count, b.hist ? b.hist : hist, b.passes,
                                                     b.plan, status, tiles, kThreads * ipt);
   for (uint32_t p = 0; p < b.passes; ++p) {
     uint32_t *st = status + (size_t)p * tiles * 256;
     constexpr int kSmall = GSR_SORT_MIN_BLOCKS, kLarge = GSR_SORT_MIN_BLOCKS_LARGE;
     if (ipt == 8) {
-      const uint32_t g = std::min(grid, resident_pass_blocks<8, kSmall>());
+      const uint32_t g = std::min(grid, resident_blocks<pass_kernel<8, kSmall>>());
       pass_kernel<8, kSmall><<<g, kThreads, 0, stream>>>(b.plan, p, b.begin_bit + 8 * p, b.keys0,
                                                          b.vals0, b.keys1, b.vals1, st,
                                                          tickets + p, b.error);
     } else if (expected < kHugeSort) {
-      const uint32_t g = std::min(grid, resident_pass_blocks<kIptLarge, kLarge>());
+      const uint32_t g = std::min(grid, resident_blocks<pass_kernel<kIptLarge, kLarge>>());
       pass_kernel<kIptLarge, kLarge><<<g, kThreads, 0, stream>>>(
           b.plan, p, b.begin_bit + 8 * p, b.keys0, b.vals0, b.keys1, b.vals1, st, tickets + p,
           b.error);
     } else {
-      const uint32_t g = std::min(grid, resident_pass_blocks<kIptLarge, 4>());
+      const uint32_t g = std::min(grid, resident_blocks<pass_kernel<kIptLarge, 4>>());
       pass_kernel<kIptLarge, 4><<<g, kThreads, 0, stream>>>(b.plan, p, b.begin_bit + 8 * p,
                                                             b.keys0, b.vals0, b.keys1, b.vals1,
                                                             st, tickets + p, b.error);

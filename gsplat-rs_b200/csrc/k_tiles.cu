@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EmitBuffers b) {
   __shared__ uint2 s_rect[kEmitItems];
   __shared__ uint16_t s_vi[kEmitItems];
   __shared__ uint32_t s_wsum[kEmitWarps];
-  __shared__ uint32_t s_hist[3][256];
+  __shared__ uint32_t s_hist[4 * 256];  // [passes][256], or one wide pass's
   __shared__ uint32_t s_block;
   __shared__ unsigned long long s_prefix;
   // View table columns: splat base, bin base, bins per row; tile pairs of the
@@ -142,7 +142,9 @@ __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EmitBuffers b) {
   uint32_t *s_vsb = s_views, *s_vbb = s_views + b.num_views, *s_vbx = s_views + 2 * b.num_views;
   uint32_t *s_vpairs = s_views + 3 * b.num_views;
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (uint32_t k = tid; k < 3 * 256; k += kEmitThreads) (&s_hist[0][0])[k] = 0;
+  const uint32_t hist_words = b.wide_bits ? 1u << b.wide_bits : b.bin_passes * 256;
+  const uint32_t low_mask = b.wide_bits ? hist_words - 1u : 255u;
+  for (uint32_t k = tid; k < hist_words; k += kEmitThreads) s_hist[k] = 0;
   for (uint32_t v = tid; v < b.num_views; v += kEmitThreads) {
     s_vsb[v] = b.views[v].splat_base;
     s_vbb[v] = b.views[v].bin_base;
@@ -295,7 +297,7 @@ __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EmitBuffers b) {
         const uint32_t t = bj + bc;
         b.pair_keys[g] = (t << kBinCodeBits) | bin_code(rows4, bc);
         b.pair_vals[g] = idj;
-        atomicAdd(&s_hist[0][t & 255u], 1u);
+        atomicAdd(&s_hist[t & low_mask], 1u);
         // The higher digits of a round's bins are mostly equal: one add per
         // distinct digit instead of up to 32 colliding ones.
         const uint32_t act = __activemask();
@@ -303,12 +305,12 @@ __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EmitBuffers b) {
         if (b.bin_passes > 1) {
           const uint32_t d1 = (t >> 8) & 255u;
           const uint32_t peers = __match_any_sync(act, d1);
-          if ((peers & lt) == 0) atomicAdd(&s_hist[1][d1], __popc(peers));
+          if ((peers & lt) == 0) atomicAdd(&s_hist[256 + d1], __popc(peers));
         }
         if (b.bin_passes > 2) {
           const uint32_t d2 = (t >> 16) & 255u;
           const uint32_t peers = __match_any_sync(act, d2);
-          if ((peers & lt) == 0) atomicAdd(&s_hist[2][d2], __popc(peers));
+          if ((peers & lt) == 0) atomicAdd(&s_hist[512 + d2], __popc(peers));
         }
       }
     }
@@ -320,8 +322,8 @@ __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EmitBuffers b) {
   if (b.num_views > 1)
     for (uint32_t v = tid; v < b.num_views; v += kEmitThreads)
       if (const uint32_t n = s_vpairs[v]) atomicAdd(&b.view_counters[v].pairs, n);
-  for (uint32_t q = tid; q < b.bin_passes * 256; q += kEmitThreads) {
-    const uint32_t n = (&s_hist[0][0])[q];
+  for (uint32_t q = tid; q < hist_words; q += kEmitThreads) {
+    const uint32_t n = s_hist[q];
     if (n) atomicAdd(&b.bin_hist[q], n);
   }
 }

@@ -63,6 +63,9 @@ struct SortBuffers {
   // Items to tune the tiles for where far fewer than `capacity` are likely
   // (0: capacity). Any count up to the capacity is sorted.
   uint32_t expected = 0;
+  // 9 or 10: one pass over that many bits (passes = 1, histograms given, and
+  // sort_work_words of 4 passes).
+  uint32_t wide_bits = 0;
 };
 constexpr uint32_t kSortScratchHeadWords = 64 + 4 * 256;  // tickets and histograms
 uint64_t sort_work_words(uint32_t capacity, uint32_t passes);
@@ -83,8 +86,10 @@ struct EmitBuffers {
   unsigned long long *status;      // [emit_blocks(n)] look-back words, zeroed
   FrameCounters *counters;
   ViewCounters *view_counters;     // pairs zeroed
-  uint32_t *bin_hist;              // [passes][256] digit histograms of the bin ids, zeroed
+  uint32_t *bin_hist;              // digit histograms of the bin ids, zeroed: [passes][256], or
+                                   // [1 << wide_bits] of one wide pass
   uint32_t bin_passes;
+  uint32_t wide_bits;
   uint32_t n;                      // total splats over the views (upper bound of visible)
   const ViewDev *views;
   uint32_t num_views;              // at most kMaxViewsPerLaunch

@@ -64,11 +64,22 @@ void DeviceBuffer::reset(uint64_t bytes) {
   bytes_ = bytes;
 }
 
-uint32_t bin_sort_passes(uint32_t num_bins) {
+namespace {
+uint32_t bits_below(uint32_t values) {  // bits that hold 0 .. values-1
   uint32_t bits = 0;
-  while (bits < 32 && (1ull << bits) < num_bins) ++bits;
-  return std::max(1u, (bits + 7) / 8);
+  while (bits < 32 && (1ull << bits) < values) ++bits;
+  return bits;
 }
+// The bin sort: one pass of up to 10 bits, else 8-bit passes.
+uint32_t bin_wide_bits(uint32_t num_bins) {
+  const uint32_t bits = bits_below(num_bins);
+  return bits == 9 || bits == 10 ? bits : 0u;
+}
+uint32_t bin_sort_passes(uint32_t num_bins) {
+  if (bin_wide_bits(num_bins)) return 1;
+  return std::max(1u, (bits_below(num_bins) + 7) / 8);
+}
+}  // namespace
 
 uint64_t scene_device_bytes(uint64_t splats, uint32_t sh_degree) {
   const uint64_t n = std::max<uint64_t>(splats, 1);
@@ -364,7 +375,7 @@ void Pipeline::ensure_workspace(const Layout &l) {
 }
 
 void Pipeline::ensure_key_workspace(uint64_t capacity) {
-  const uint32_t passes = 3;  // enough for any bin count
+  const uint32_t passes = 4;  // enough for any bin count (a wide pass takes as many words)
   if (key_cap_ >= capacity && key_ws_.get()) return;
   if (capacity > kMaxSortItems)
     throw Error(Code::Unsupported, "tile pair count " + std::to_string(capacity) +
@@ -439,8 +450,8 @@ void Pipeline::launch_all(const Layout &l, uint32_t *images, const HostSinks &si
 
   EmitBuffers eb{depth_plan_, vis_vals0_,  vis_vals1_, rects_,        records_,
                  pair_keys0_, pair_vals0_, key_cap_,   emit_status_,  counters_,
-                 view_counters_, bin_hist_, l.bin_passes, l.total_splats, views_dev,
-                 l.views, tile_};
+                 view_counters_, bin_hist_, l.bin_passes, bin_wide_bits(l.total_bins),
+                 l.total_splats, views_dev, l.views, tile_};
   launch_emit(eb, stream_);
   if (debug_) {
     GSR_CUDA(cudaMemcpyAsync(debug_pairs_.as<uint32_t>(), pair_keys0_, 4 * key_cap_,
@@ -453,6 +464,7 @@ void Pipeline::launch_all(const Layout &l, uint32_t *images, const HostSinks &si
                  (uint32_t)key_cap_, kBinCodeBits, l.bin_passes, bin_plan_, pair_sort_work_,
                  &counters_->error, bin_hist_, true};
   ts.expected = std::max<uint32_t>((uint32_t)(key_cap_ / kPairsPerBinPair), 1);
+  ts.wide_bits = bin_wide_bits(l.total_bins);
   launch_sort(ts, stream_);
   record(4);
   launch_ranges(bin_plan_, pair_keys0_, pair_keys1_, counters_, (uint32_t)key_cap_, ranges_,

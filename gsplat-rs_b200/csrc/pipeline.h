@@ -360,6 +360,5 @@ class Pipeline {
   uint64_t graph_clock_ = 0;
 };
 
-uint32_t bin_sort_passes(uint32_t num_tiles);
 
 }  // namespace gsr

@@ -54,3 +54,18 @@ def test_views_past_the_bins_of_one_run():
             ctx = _render(scene, cams[k], 16384, 8, tile=8, debug=False)
             assert np.array_equal(b.readback_rgba8(k), ctx.readback_rgba8()), k
             assert b.view_stats(k).tile_pairs == ctx.frame_counts().tile_keys
+
+
+@pytest.mark.parametrize("w,h,tile", [
+    (1100, 1000, 16),  # 288 bins: one pass of 512 digits
+    (2048, 128, 8),    # 256 bins: the last of one 8-bit pass
+    (700, 900, 8),     # 638 bins: one pass of 1,024 digits
+    (1024, 1024, 8),   # 1,024 bins: the last of it
+    (1100, 1000, 8)])  # 1,120 bins: two 8-bit passes
+def test_bin_sort_digits(oracle, w, h, tile):
+    """The tile lists over every kind of bin sort, with several sort tiles."""
+    scene, cam = _scene(30_000, 40)
+    sv = oracle.SceneView(scene)
+    fr = oracle.Frame(sv, cam, w, h, tile=tile)
+    ctx = _render(scene, cam, w, h, tile=tile)
+    _compare_stages(ctx, fr, sv)
