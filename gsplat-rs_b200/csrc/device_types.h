@@ -103,7 +103,7 @@ struct ViewSetDev {
   uint32_t first_view;  // index into the view table
   uint32_t count;       // 1..kMaxSetViews
   uint32_t block_base;  // first preprocess block of the set
-  uint32_t pad;
+  uint32_t key_base;    // first key block
 };
 constexpr uint32_t kMaxSetViews = 16;
 

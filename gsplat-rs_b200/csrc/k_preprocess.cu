@@ -4,15 +4,19 @@
 // bit (division and sqrt are IEEE-rounded; there are no transcendental calls
 // per frame — alpha, extent scale and covariance are precomputed at load).
 //
-// One thread per splat:
+// Two kernels, since only the first stands before the depth sort:
+//   keys_kernel:
 //   1. depth = row2 . (p - cam); visible iff near <= depth <= far
 //      (preprocess_visible_into, crates/gsplat-render-wgpu/src/lib.rs:1263-1296);
-//   2. project_splat + eval_color (splat_surface_direct.wgsl:131-217, 233-334),
-//      tile rect of the ellipse |local| <= s and the pixel-space record;
-//   3. digit histograms of the depth keys for the radix sort;
-//   4. visible splats are compacted in id order with a block scan and a
+//   2. digit histograms of the depth keys for the radix sort;
+//   3. visible splats are compacted in id order with a block scan and a
 //      decoupled look-back, emitting (~bits(max(depth, 0)), id) so that an
 //      ascending stable sort yields the reference's descending-depth order.
+//   preprocess_kernel, beside the depth sort: project_splat + eval_color
+//      (splat_surface_direct.wgsl:131-217, 233-334), the tile rect of the
+//      ellipse |local| <= s and the pixel-space record of every visible splat.
+// As one kernel the vertex stage waited for the ordered compaction (a third of
+// a warp's time) and the sort for the vertex stage.
 
 #include "device_common.cuh"
 #include "kernels.h"
@@ -302,6 +306,15 @@ struct PackedIn {
   float ext;          // the extent scale of the opacity code
 };
 
+// Position from the first two words of a hot record; h: the scene's header
+// (bounds min, span).
+__device__ __forceinline__ void packed_position(uint32_t w0, uint32_t w1, const float *h, float &x,
+                                                float &y, float &z) {
+  x = h[0] + div_const((float)(w0 & 0xffffu), 65535.0f, 1.0f / 65535.0f) * h[3];
+  y = h[1] + div_const((float)(w0 >> 16), 65535.0f, 1.0f / 65535.0f) * h[4];
+  z = h[2] + div_const((float)(w1 & 0xffffu), 65535.0f, 1.0f / 65535.0f) * h[5];
+}
+
 template <int kPlanes>
 __device__ __forceinline__ void decode_packed(uint32_t planes, const PackedIn &in,
                                               K1Stage<kPlanes> &st) {
@@ -309,11 +322,8 @@ __device__ __forceinline__ void decode_packed(uint32_t planes, const PackedIn &i
   const uint32_t *side = in.side;
   const float *h = in.h;
   const uint32_t t = threadIdx.x;
-  const uint32_t pu[3] = {w[0] & 0xffffu, w[0] >> 16, w[1] & 0xffffu};
   float pos[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-    pos[a] = h[a] + div_const((float)pu[a], 65535.0f, 1.0f / 65535.0f) * h[3 + a];
+  packed_position(w[0], w[1], h, pos[0], pos[1], pos[2]);
   const uint32_t op = (w[1] >> 16) & 0xffu;
   const float alpha = fminf(fmaxf(div_const((float)op, 255.0f, 1.0f / 255.0f), 1e-4f), 1.0f - 1e-4f);
   st.pos[t] = make_float4(pos[0], pos[1], pos[2], alpha);
@@ -368,38 +378,184 @@ __device__ __forceinline__ void decode_packed(uint32_t planes, const PackedIn &i
                                     coeff(4 * pl + 3));
 }
 
+// ---- depth keys --------------------------------------------------------------
+
+// Splats per thread of the key kernel: 1,024 a block, few enough blocks for a
+// short look-back (256 a block: 16k splats 4 us slower, 64 thumbnail views of
+// 16k the same).
+constexpr int kKeyItems = 4;
+constexpr uint32_t kKeyTile = kK1Threads * kKeyItems;
+
+// The views a block handles: their uniforms and splat bases, in shared memory.
+struct SetViews {
+  FrameParams p[kMaxSetViews];
+  uint32_t base[kMaxSetViews];
+
+  __device__ __forceinline__ void load(const ViewDev *views, const ViewSetDev &set) {
+    constexpr uint32_t kWords = sizeof(FrameParams) / 4;
+    static_assert(sizeof(FrameParams) % 4 == 0, "FrameParams is copied as words");
+    for (uint32_t w = threadIdx.x; w < set.count * kWords; w += kK1Threads) {
+      const uint32_t v = w / kWords, o = w % kWords;
+      reinterpret_cast<uint32_t *>(&p[v])[o] =
+          reinterpret_cast<const uint32_t *>(&views[set.first_view + v].p)[o];
+    }
+    if (threadIdx.x < set.count) base[threadIdx.x] = views[set.first_view + threadIdx.x].splat_base;
+  }
+};
+
+// Depth of position (x, y, z) in a view, and whether it is visible.
+__device__ __forceinline__ bool view_depth(const FrameParams &p, float x, float y, float z,
+                                           float &depth) {
+  const float rx = x - p.cam[0], ry = y - p.cam[1], rz = z - p.cam[2];
+  depth = p.r2[0] * rx + p.r2[1] * ry + p.r2[2] * rz;
+  return depth >= p.near_plane && depth <= p.far_plane;
+}
+
+// One block covers kKeyTile consecutive splats of one scene for every view of a
+// view set. Visible entries are compacted in (block, view, id) order, which
+// keeps every view's entries in ascending id order.
+__global__ void __launch_bounds__(kK1Threads)
+    keys_kernel(const ViewDev *__restrict__ views, const ViewSetDev *__restrict__ sets,
+                uint32_t num_sets, uint32_t total_blocks, K1Buffers b) {
+  __shared__ uint32_t s_block;
+  __shared__ ViewSetDev s_set;
+  __shared__ uint32_t s_cnt[kMaxSetViews][kK1Warps];  // visible per view and warp
+  __shared__ uint32_t s_hist[4][256];
+  __shared__ SetViews s_views;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool one_set = num_sets == 1;
+  if (threadIdx.x == 0) {
+    ViewSetDev set0 = sets[0];  // read beside the ticket
+    const uint32_t blk = atomicAdd(&b.counters->k1_ticket, 1u);
+    if (!one_set)
+      set0 = sets[find_view(num_sets, blk, [&](uint32_t v) { return sets[v].key_base; })];
+    s_block = blk;
+    s_set = set0;
+  }
+  if (one_set) s_views.load(views, sets[0]);
+  for (uint32_t k = threadIdx.x; k < 4 * 256; k += kK1Threads) (&s_hist[0][0])[k] = 0;
+  __syncthreads();
+  const uint32_t block = s_block;
+  const ViewSetDev set = s_set;
+  if (!one_set) {
+    s_views.load(views, set);
+    __syncthreads();
+  }
+  const SceneDev &sc = views[set.first_view].sc;
+  const uint32_t n = sc.n;
+  // item j of lane l: splat (block, warp, j, l)
+  const uint32_t i0 = (block - set.key_base) * kKeyTile + warp * (32 * kKeyItems) + lane;
+  float x[kKeyItems], y[kKeyItems], z[kKeyItems];
+#pragma unroll
+  for (int j = 0; j < kKeyItems; ++j) {
+    const uint32_t i = i0 + 32 * j;
+    x[j] = y[j] = z[j] = 0.0f;
+    if (i >= n) continue;
+    if (sc.hot) {
+      packed_position(sc.hot[5 * (size_t)i], sc.hot[5 * (size_t)i + 1], sc.packed, x[j], y[j],
+                      z[j]);
+    } else {
+      const float4 pa = sc.pos_alpha[i];
+      x[j] = pa.x;
+      y[j] = pa.y;
+      z[j] = pa.z;
+    }
+  }
+  for (uint32_t k = 0; k < set.count; ++k) {
+    uint32_t count = 0;
+#pragma unroll
+    for (int j = 0; j < kKeyItems; ++j) {
+      float depth;
+      const bool vis = view_depth(s_views.p[k], x[j], y[j], z[j], depth) && i0 + 32 * j < n;
+      count += __popc(__ballot_sync(0xffffffffu, vis));
+    }
+    if (lane == 0) s_cnt[k][warp] = count;
+  }
+  __syncthreads();
+  uint32_t block_total = 0;
+  for (uint32_t k = 0; k < set.count; ++k)
+#pragma unroll
+    for (int w = 0; w < kK1Warps; ++w) block_total += s_cnt[k][w];
+  if (threadIdx.x < set.count) {
+    uint32_t c = 0;
+#pragma unroll
+    for (int w = 0; w < kK1Warps; ++w) c += s_cnt[threadIdx.x][w];
+    if (c) atomicAdd(&b.view_counters[set.first_view + threadIdx.x].visible, c);
+  }
+  if (b.reuse_order) {  // only counted
+    if (threadIdx.x == 0) atomicAdd(&b.counters->visible, block_total);
+    return;
+  }
+  if (threadIdx.x == 0) lookback_publish_aggregate(b.status, block, block_total);
+  // Every warp resolves the block's offset on its own (no second block
+  // barrier); warp 0 publishes the inclusive prefix.
+  const unsigned long long prefix = lookback_resolve(b.status, block, &b.counters->error);
+  if (warp == 0 && lane == 0) {
+    lookback_publish_inclusive(b.status, block, prefix + block_total);
+    if (block == total_blocks - 1) b.counters->visible = (uint32_t)(prefix + block_total);
+  }
+  uint32_t slot = (uint32_t)prefix;
+  for (uint32_t k = 0; k < set.count; ++k) {
+    uint32_t at = slot;
+#pragma unroll
+    for (int w = 0; w < kK1Warps; ++w) {
+      const uint32_t c = s_cnt[k][w];
+      at += (w < (int)warp) ? c : 0u;
+      slot += c;
+    }
+#pragma unroll
+    for (int j = 0; j < kKeyItems; ++j) {
+      const uint32_t i = i0 + 32 * j;
+      float depth;
+      const bool vis = view_depth(s_views.p[k], x[j], y[j], z[j], depth) && i < n;
+      const uint32_t bal = __ballot_sync(0xffffffffu, vis);
+      if (vis) {
+        const uint32_t key = ~__float_as_uint(fmaxf(depth, 0.0f));
+        const uint32_t to = at + __popc(bal & lanemask_lt());
+        b.vis_keys[to] = key;
+        b.vis_ids[to] = s_views.base[k] + i;
+        // Digit histograms for every radix pass.
+#pragma unroll
+        for (int d = 0; d < 4; ++d) atomicAdd(&s_hist[d][(key >> (8 * d)) & 255u], 1u);
+      }
+      at += __popc(bal);
+    }
+  }
+  __syncthreads();
+  for (uint32_t k = threadIdx.x; k < 4 * 256; k += kK1Threads) {
+    const uint32_t c = (&s_hist[0][0])[k];
+    if (c) atomicAdd(&b.key_hist[k], c);
+  }
+}
+
+// ---- vertex stage ------------------------------------------------------------
+
 // One block covers 256 consecutive splats of one scene for every view of a
 // view set (up to kMaxSetViews views of that scene). One thread stages the
 // block's slice of every scene plane into shared memory with bulk copies
 // (cp.async.bulk, completion on an mbarrier), so all of the block's HBM
 // reads are in flight at once and every view of the set reads the slice
-// from shared memory: the scene is read from HBM once per set. Positions
-// arrive on their own barrier, so the depth tests start while covariance and
-// colour are still in flight. Per view, the arithmetic is exactly the
-// single-view sequence. Visible entries are compacted in (block, view, id)
-// order, which keeps every view's entries in ascending id order.
+// from shared memory: the scene is read from HBM once per set. Per view, the
+// arithmetic is exactly the single-view sequence.
 template <int kPlanes, bool kDebug>
 __global__ void __launch_bounds__(kK1Threads, GSR_K1_MIN_BLOCKS)
     preprocess_kernel(const ViewDev *__restrict__ views, const ViewSetDev *__restrict__ sets,
-                      uint32_t num_sets, uint32_t total_blocks, K1Buffers b) {
+                      uint32_t num_sets, K1Buffers b) {
   extern __shared__ __align__(128) unsigned char k1_dyn[];
   K1Stage<kPlanes> &st = *reinterpret_cast<K1Stage<kPlanes> *>(k1_dyn);
-  __shared__ uint32_t s_block;
-  __shared__ uint32_t s_set;
+  __shared__ ViewSetDev s_set;
   __shared__ uint32_t s_lost;  // a stage wait expired twice: copies may still land
-  __shared__ uint32_t s_cnt[kMaxSetViews][kK1Warps];  // visible per view and warp
-  __shared__ uint32_t s_hist[4][256];
-  __shared__ FrameParams s_params[kMaxSetViews];  // the set's per-view uniforms
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ SetViews s_views;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t block = blockIdx.x;
+  const bool one_set = num_sets == 1;
   if (threadIdx.x == 0) {
-    const uint32_t blk = atomicAdd(&b.counters->k1_ticket, 1u);
-    s_block = blk;
+    const ViewSetDev set0 =
+        sets[find_view(num_sets, block, [&](uint32_t v) { return sets[v].block_base; })];
+    s_set = set0;
     s_lost = 0;
-    const uint32_t si = find_view(num_sets, blk, [&](uint32_t v) { return sets[v].block_base; });
-    s_set = si;
-    const ViewSetDev set0 = sets[si];
     const SceneDev sc0 = views[set0.first_view].sc;
-    const uint32_t i0 = (blk - set0.block_base) * kK1Threads;
+    const uint32_t i0 = (block - set0.block_base) * kK1Threads;
     const uint32_t bytes = min((uint32_t)kK1Threads, sc0.n - i0) * 16u;  // >= 16: i0 < n
     mbar_init(&st.bar[0], 1);
     mbar_init(&st.bar[1], 1);
@@ -425,20 +581,13 @@ __global__ void __launch_bounds__(kK1Threads, GSR_K1_MIN_BLOCKS)
         bulk_copy_g2s(st.color[q], sc0.color + (size_t)q * sc0.n + i0, bytes, &st.bar[1]);
     }
   }
-  for (uint32_t k = threadIdx.x; k < 4 * 256; k += kK1Threads) (&s_hist[0][0])[k] = 0;
+  if (one_set) s_views.load(views, sets[0]);
   __syncthreads();
-  const uint32_t block = s_block;
-  const ViewSetDev set = sets[s_set];
-  {
-    constexpr uint32_t kWords = sizeof(FrameParams) / 4;
-    static_assert(sizeof(FrameParams) % 4 == 0, "FrameParams is copied as words");
-    for (uint32_t w = threadIdx.x; w < set.count * kWords; w += kK1Threads) {
-      const uint32_t v = w / kWords, o = w % kWords;
-      reinterpret_cast<uint32_t *>(&s_params[v])[o] =
-          reinterpret_cast<const uint32_t *>(&views[set.first_view + v].p)[o];
-    }
+  const ViewSetDev set = s_set;
+  if (!one_set) {
+    s_views.load(views, set);
+    __syncthreads();
   }
-  __syncthreads();
   const SceneDev sc = views[set.first_view].sc;
   const uint32_t i = (block - set.block_base) * kK1Threads + threadIdx.x;
   const bool valid = i < sc.n;
@@ -485,32 +634,6 @@ __global__ void __launch_bounds__(kK1Threads, GSR_K1_MIN_BLOCKS)
   }
   const float4 pa = valid && ok0 ? st.pos[threadIdx.x] : make_float4(0.f, 0.f, 0.f, 0.f);
 
-  // Depth test for every view of the set. The block's visible count is
-  // known right after it: publish it for the successors' look-back before
-  // doing the heavy vertex stage.
-  uint32_t vis_bits = 0;
-  for (uint32_t k = 0; k < set.count; ++k) {
-    const FrameParams &p = s_params[k];
-    const float rx = pa.x - p.cam[0], ry = pa.y - p.cam[1], rz = pa.z - p.cam[2];
-    const float depth = p.r2[0] * rx + p.r2[1] * ry + p.r2[2] * rz;
-    const bool vis = valid && ok0 && depth >= p.near_plane && depth <= p.far_plane;
-    const uint32_t ballot = __ballot_sync(0xffffffffu, vis);
-    if (lane == 0) s_cnt[k][warp] = __popc(ballot);
-    vis_bits |= (vis ? 1u : 0u) << k;
-  }
-  __syncthreads();
-  uint32_t block_total = 0;
-  for (uint32_t k = 0; k < set.count; ++k)
-#pragma unroll
-    for (int w = 0; w < kK1Warps; ++w) block_total += s_cnt[k][w];
-  if (threadIdx.x == 0) lookback_publish_aggregate(b.status, block, block_total);
-  if (threadIdx.x < set.count) {
-    uint32_t c = 0;
-#pragma unroll
-    for (int w = 0; w < kK1Warps; ++w) c += s_cnt[threadIdx.x][w];
-    if (c) atomicAdd(&b.view_counters[set.first_view + threadIdx.x].visible, c);
-  }
-
   if (!sc.hot) {
     ok1 = mbar_wait(&st.bar[1], 0, &b.counters->error) || mbar_wait(&st.bar[1], 0, &b.counters->error);
     if (!ok1) s_lost = 1;
@@ -520,12 +643,11 @@ __global__ void __launch_bounds__(kK1Threads, GSR_K1_MIN_BLOCKS)
   const float4 cb = ok1 ? st.cov_b[threadIdx.x] : zero4;
   const float4 *col = &st.color[0][threadIdx.x];
   for (uint32_t k = 0; k < set.count; ++k) {
-    const uint32_t view = set.first_view + k;
-    const FrameParams &p = s_params[k];
-    const uint32_t gid = views[view].splat_base + i;
-    const bool vis = (vis_bits >> k) & 1u;
-    float rel[3] = {pa.x - p.cam[0], pa.y - p.cam[1], pa.z - p.cam[2]};
-    const float depth = p.r2[0] * rel[0] + p.r2[1] * rel[1] + p.r2[2] * rel[2];
+    const FrameParams &p = s_views.p[k];
+    const uint32_t gid = s_views.base[k] + i;
+    const float rel[3] = {pa.x - p.cam[0], pa.y - p.cam[1], pa.z - p.cam[2]};
+    float depth;
+    const bool vis = view_depth(p, pa.x, pa.y, pa.z, depth) && valid;
     ProjectedDev *dbg = nullptr;
     if (kDebug && valid) {
       dbg = &b.projected[gid];
@@ -535,20 +657,13 @@ __global__ void __launch_bounds__(kK1Threads, GSR_K1_MIN_BLOCKS)
       *dbg = z;
     }
     bool drawn = false;
-    // Digit histograms of the depth keys for every radix pass (every
-    // compacted key is counted).
-    if (vis && !b.reuse_order) {
-      const uint32_t key = ~__float_as_uint(fmaxf(depth, 0.0f));
-#pragma unroll
-      for (int d = 0; d < 4; ++d) atomicAdd(&s_hist[d][(key >> (8 * d)) & 255u], 1u);
-    }
-    if (vis && ok1) {
+    if (vis && ok0 && ok1) {
       Record rec;
       uint2 rect = make_uint2(0u, 0u);
       drawn = project<kPlanes>(p, pa, ca, cb, col, rel, depth, rec, rect, dbg);
       b.rects[gid] = rect;
       if (drawn) b.records[gid] = rec;
-    } else if ((b.reuse_order || vis) && valid) {
+    } else if ((b.reuse_order || vis || !ok0) && valid) {
       // The reused order may list this splat (or its stage was lost): it
       // emits no tile this frame.
       b.rects[gid] = make_uint2(0u, 0u);
@@ -556,62 +671,42 @@ __global__ void __launch_bounds__(kK1Threads, GSR_K1_MIN_BLOCKS)
     const uint32_t dmask = __ballot_sync(0xffffffffu, drawn);
     if (lane == 0 && dmask) {
       atomicAdd(&b.counters->drawn, __popc(dmask));
-      atomicAdd(&b.view_counters[view].drawn, __popc(dmask));
+      atomicAdd(&b.view_counters[set.first_view + k].drawn, __popc(dmask));
     }
-  }
-
-  // Every warp resolves the block's offset on its own (no second block
-  // barrier); warp 0 publishes the inclusive prefix.
-  const unsigned long long prefix = lookback_resolve(b.status, block, &b.counters->error);
-  if (warp == 0 && lane == 0) {
-    lookback_publish_inclusive(b.status, block, prefix + block_total);
-    if (block == total_blocks - 1) b.counters->visible = (uint32_t)(prefix + block_total);
-  }
-  uint32_t slot = (uint32_t)prefix;
-  for (uint32_t k = 0; k < set.count; ++k) {
-    uint32_t warp_prefix = 0, view_total = 0;
-#pragma unroll
-    for (int w = 0; w < kK1Warps; ++w) {
-      const uint32_t c = s_cnt[k][w];
-      warp_prefix += (w < (int)warp) ? c : 0u;
-      view_total += c;
-    }
-    const bool vis = (vis_bits >> k) & 1u;
-    const uint32_t bal = __ballot_sync(0xffffffffu, vis);
-    if (vis && !b.reuse_order) {
-      const uint32_t view = set.first_view + k;
-      const FrameParams &p = s_params[k];
-      const float rx = pa.x - p.cam[0], ry = pa.y - p.cam[1], rz = pa.z - p.cam[2];
-      const float depth = p.r2[0] * rx + p.r2[1] * ry + p.r2[2] * rz;
-      const uint32_t at = slot + warp_prefix + __popc(bal & lanemask_lt());
-      b.vis_keys[at] = ~__float_as_uint(fmaxf(depth, 0.0f));
-      b.vis_ids[at] = views[view].splat_base + i;
-    }
-    slot += view_total;
   }
   __syncthreads();
   if (threadIdx.x == 0 && !s_lost) {  // every thread has passed both waits
     mbar_inval(&st.bar[0]);
     mbar_inval(&st.bar[1]);
   }
-  for (uint32_t k = threadIdx.x; k < 4 * 256; k += kK1Threads) {
-    uint32_t c = (&s_hist[0][0])[k];
-    if (c) atomicAdd(&b.key_hist[k], c);
-  }
 }
+
+// A frame's depth sort has about a block an SM (2,048 keys each), and each of
+// its passes waits for room beside the vertex stage, whose three blocks take
+// an SM's registers. Up to kTwoBlockTiles blocks the vertex stage asks for so
+// much shared memory that two fit and a sort block beside them (279k splats:
+// both together 73 -> 69 us); longer ones take all three (3M: 318 us against
+// 326, 1.0 M packed 146 against 151).
+constexpr size_t kTwoBlockSmem = 78'000;
+constexpr uint32_t kTwoBlockTiles = 1600;
 
 template <int kPlanes, bool kDebug>
 void launch_k1_t(const ViewDev *views, const ViewSetDev *sets, uint32_t num_sets,
                  uint32_t total_blocks, const K1Buffers &b, cudaStream_t stream) {
   constexpr size_t kSmem = sizeof(K1Stage<kPlanes>);
+  constexpr size_t kMost = kSmem > kTwoBlockSmem ? kSmem : kTwoBlockSmem;
   static const bool configured = [] {
     cudaFuncSetAttribute(preprocess_kernel<kPlanes, kDebug>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost);
+    cudaFuncSetAttribute(preprocess_kernel<kPlanes, kDebug>,
+                         cudaFuncAttributePreferredSharedMemoryCarveout,
+                         cudaSharedmemCarveoutMaxShared);
     return true;
   }();
   (void)configured;
+  const size_t smem = total_blocks <= kTwoBlockTiles && !b.reuse_order ? kMost : kSmem;
   preprocess_kernel<kPlanes, kDebug>
-      <<<total_blocks, kK1Threads, kSmem, stream>>>(views, sets, num_sets, total_blocks, b);
+      <<<total_blocks, kK1Threads, smem, stream>>>(views, sets, num_sets, b);
 }
 
 template <int kPlanes>
@@ -625,6 +720,14 @@ void launch_k1(const ViewDev *views, const ViewSetDev *sets, uint32_t num_sets,
 }
 
 }  // namespace
+
+uint32_t key_blocks(uint32_t splats) { return (splats + kKeyTile - 1) / kKeyTile; }
+
+void launch_keys(const ViewDev *views, const ViewSetDev *sets, uint32_t num_sets,
+                 uint32_t total_blocks, const K1Buffers &b, cudaStream_t stream) {
+  if (total_blocks == 0) return;
+  keys_kernel<<<total_blocks, kK1Threads, 0, stream>>>(views, sets, num_sets, total_blocks, b);
+}
 
 uint32_t preprocess_blocks(uint32_t splats) { return (splats + kK1Threads - 1) / kK1Threads; }
 

@@ -632,18 +632,35 @@ uint32_t device_sm_count() {
 }
 
 namespace {
+// Launches a kernel of the sort at the sort's priority. The priority of a
+// captured launch is the launch's own, not its stream's.
+template <typename... P, typename... A>
+void launch_at(const SortBuffers &b, void (*kernel)(P...), uint32_t grid, cudaStream_t stream,
+               A... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(kThreads);
+  c.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributePriority;
+  attr.val.priority = b.priority;
+  c.attrs = &attr;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // The one pass of a wide sort; the histograms are given.
 template <int kBits>
 void launch_wide(const SortBuffers &b, cudaStream_t stream) {
   constexpr uint32_t kTile = kThreads * kWideIpt;
   const uint32_t tiles = std::max<uint32_t>((uint32_t)(((uint64_t)b.capacity + kTile - 1) / kTile), 1);
   uint32_t *status = b.work + kSortScratchHeadWords;
-  plan_kernel<(1 << kBits) / kThreads>
-      <<<std::min<uint32_t>(tiles, 2 * device_sm_count()), kThreads, 0, stream>>>(
-          b.count, b.hist, 1, b.plan, status, tiles, kTile);
+  launch_at(b, plan_kernel<(1 << kBits) / kThreads>,
+            std::min<uint32_t>(tiles, 2 * device_sm_count()), stream, b.count, b.hist, 1, b.plan,
+            status, tiles, kTile);
   const uint32_t grid = std::min(tiles, resident_blocks<wide_kernel<kBits>>());
-  wide_kernel<kBits><<<grid, kThreads, 0, stream>>>(b.plan, b.begin_bit, b.keys0, b.vals0,
-                                                    b.keys1, b.vals1, status, b.work, b.error);
+  launch_at(b, wide_kernel<kBits>, grid, stream, b.plan, b.begin_bit, b.keys0, b.vals0, b.keys1,
+            b.vals1, status, b.work, b.error);
 }
 }  // namespace
 
@@ -667,27 +684,21 @@ void launch_sort(const SortBuffers &b, cudaStream_t stream) {
           <<<grid, kThreads, 0, stream>>>(b.keys0, b.count, b.begin_bit, b.passes, hist);
   }
   const uint32_t zero_blocks = std::min<uint32_t>(grid, 2 * device_sm_count());
-  plan_kernel<1><<<zero_blocks, kThreads, 0, stream>>>(b.count, b.hist ? b.hist : hist, b.passes,
-                                                    b.plan, status, tiles, kThreads * ipt);
+  launch_at(b, plan_kernel<1>, zero_blocks, stream, b.count, b.hist ? b.hist : hist, b.passes,
+            b.plan, status, tiles, kThreads * ipt);
+  constexpr int kSmall = GSR_SORT_MIN_BLOCKS, kLarge = GSR_SORT_MIN_BLOCKS_LARGE;
   for (uint32_t p = 0; p < b.passes; ++p) {
-    uint32_t *st = status + (size_t)p * tiles * 256;
-    constexpr int kSmall = GSR_SORT_MIN_BLOCKS, kLarge = GSR_SORT_MIN_BLOCKS_LARGE;
-    if (ipt == 8) {
-      const uint32_t g = std::min(grid, resident_blocks<pass_kernel<8, kSmall>>());
-      pass_kernel<8, kSmall><<<g, kThreads, 0, stream>>>(b.plan, p, b.begin_bit + 8 * p, b.keys0,
-                                                         b.vals0, b.keys1, b.vals1, st,
-                                                         tickets + p, b.error);
-    } else if (expected < kHugeSort) {
-      const uint32_t g = std::min(grid, resident_blocks<pass_kernel<kIptLarge, kLarge>>());
-      pass_kernel<kIptLarge, kLarge><<<g, kThreads, 0, stream>>>(
-          b.plan, p, b.begin_bit + 8 * p, b.keys0, b.vals0, b.keys1, b.vals1, st, tickets + p,
-          b.error);
-    } else {
-      const uint32_t g = std::min(grid, resident_blocks<pass_kernel<kIptLarge, 4>>());
-      pass_kernel<kIptLarge, 4><<<g, kThreads, 0, stream>>>(b.plan, p, b.begin_bit + 8 * p,
-                                                            b.keys0, b.vals0, b.keys1, b.vals1,
-                                                            st, tickets + p, b.error);
-    }
+    auto pass = [&](auto kernel, uint32_t resident) {
+      launch_at(b, kernel, std::min(grid, resident), stream, b.plan, p, b.begin_bit + 8 * p,
+                b.keys0, b.vals0, b.keys1, b.vals1, status + (size_t)p * tiles * 256,
+                tickets + p, b.error);
+    };
+    if (ipt == 8)
+      pass(pass_kernel<8, kSmall>, resident_blocks<pass_kernel<8, kSmall>>());
+    else if (expected < kHugeSort)
+      pass(pass_kernel<kIptLarge, kLarge>, resident_blocks<pass_kernel<kIptLarge, kLarge>>());
+    else
+      pass(pass_kernel<kIptLarge, 4>, resident_blocks<pass_kernel<kIptLarge, 4>>());
   }
 }
 

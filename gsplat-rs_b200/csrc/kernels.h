@@ -25,7 +25,7 @@ struct K1Buffers {
   uint32_t *vis_ids;           // [total splats] their gids, view-major then ascending id
   uint2 *rects;                // [gid] tile rect per visible splat ((0, 0): none)
   Record *records;             // [gid] raster record per drawn splat
-  unsigned long long *status;  // [total blocks] look-back words, zeroed
+  unsigned long long *status;  // [total key blocks] look-back words, zeroed
   FrameCounters *counters;
   uint32_t *key_hist;          // [4][256] digit histograms of the depth keys, zeroed
   ViewCounters *view_counters; // [views], zeroed
@@ -34,9 +34,14 @@ struct K1Buffers {
   // keys, ids or histograms, and clear the rects of splats not visible now.
   bool reuse_order;
 };
-uint32_t preprocess_blocks(uint32_t splats);  // blocks one view set of `splats` splats needs
-// One block per 256 splats of each view set (views of one scene handled
-// together); total_blocks = sum over sets of preprocess_blocks(scene splats).
+// Blocks one view set (views of one scene handled together) of `splats` splats
+// needs; total_blocks = their sum over the sets.
+uint32_t preprocess_blocks(uint32_t splats);
+uint32_t key_blocks(uint32_t splats);
+// The depth keys and ids of the visible splats, their count and histograms.
+void launch_keys(const ViewDev *views, const ViewSetDev *sets, uint32_t num_sets,
+                 uint32_t total_blocks, const K1Buffers &b, cudaStream_t stream);
+// The records and rects; independent of the keys.
 void launch_preprocess(const ViewDev *views, const ViewSetDev *sets, uint32_t num_sets,
                        uint32_t total_blocks, uint32_t max_planes, const K1Buffers &b, bool debug,
                        cudaStream_t stream);
@@ -66,6 +71,7 @@ struct SortBuffers {
   // 9 or 10: one pass over that many bits (passes = 1, histograms given, and
   // sort_work_words of 4 passes).
   uint32_t wide_bits = 0;
+  int priority = 0;  // launch priority of the kernels (as a stream's)
 };
 constexpr uint32_t kSortScratchHeadWords = 64 + 4 * 256;  // tickets and histograms
 uint64_t sort_work_words(uint32_t capacity, uint32_t passes);

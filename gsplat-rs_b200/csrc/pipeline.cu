@@ -136,6 +136,12 @@ Pipeline::Pipeline(int device, cudaStream_t stream) : device_(device), stream_(s
   sm_count_ = (uint32_t)sms;
   for (auto &ev : ev_) GSR_CUDA(cudaEventCreate(&ev));
   for (auto &ev : slot_ev_) GSR_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  int least = 0, greatest = 0;
+  GSR_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+  GSR_CUDA(cudaStreamCreateWithPriority(&side_stream_, cudaStreamNonBlocking, greatest));
+  side_priority_ = greatest;
+  GSR_CUDA(cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming));
+  GSR_CUDA(cudaEventCreateWithFlags(&join_ev_, cudaEventDisableTiming));
   GSR_CUDA(cudaMallocHost(&counters_host_, sizeof(FrameCounters)));
   std::memset(counters_host_, 0, sizeof(FrameCounters));
   // fixed scratch: [counters | key hist | tile hist] zeroed per run, then
@@ -161,8 +167,11 @@ Pipeline::Pipeline(int device, cudaStream_t stream) : device_(device), stream_(s
 
 Pipeline::~Pipeline() {
   cudaSetDevice(device_);
-  cudaStreamSynchronize(stream_);
+  cudaStreamSynchronize(stream_);  // and with it the side stream, joined in every run
   drop_graph();
+  if (side_stream_) cudaStreamDestroy(side_stream_);
+  if (fork_ev_) cudaEventDestroy(fork_ev_);
+  if (join_ev_) cudaEventDestroy(join_ev_);
   for (auto &ev : ev_)
     if (ev) cudaEventDestroy(ev);
   for (auto &ev : slot_ev_)
@@ -224,7 +233,7 @@ Pipeline::Layout Pipeline::plan_views(const ViewSpec *views, uint32_t count,
   l.views = count;
   views_host_.resize(count);
   sets_host_.clear();
-  uint64_t splats = 0, blocks = 0, tiles = 0, bins = 0;
+  uint64_t splats = 0, blocks = 0, keys = 0, tiles = 0, bins = 0;
   for (uint32_t v = 0; v < count; ++v) {
     const ViewSpec &vs = views[v];
     if (!camera_valid(vs.camera)) throw Error(Code::InvalidArgument, "invalid camera");
@@ -242,8 +251,9 @@ Pipeline::Layout Pipeline::plan_views(const ViewSpec *views, uint32_t count,
     // Consecutive views of one scene form a view set (one scene read in K1).
     if (sets_host_.empty() || views[v - 1].scene != vs.scene ||
         sets_host_.back().count == kMaxSetViews) {
-      sets_host_.push_back(ViewSetDev{v, 0, (uint32_t)blocks, 0});
+      sets_host_.push_back(ViewSetDev{v, 0, (uint32_t)blocks, (uint32_t)keys});
       blocks += preprocess_blocks(vs.scene->n);
+      keys += key_blocks(vs.scene->n);
     }
     sets_host_.back().count++;
     d.set = (uint32_t)sets_host_.size() - 1;
@@ -259,6 +269,7 @@ Pipeline::Layout Pipeline::plan_views(const ViewSpec *views, uint32_t count,
   l.total_splats = (uint32_t)splats;
   l.sets = (uint32_t)sets_host_.size();
   l.total_blocks = (uint32_t)blocks;
+  l.key_blocks = (uint32_t)keys;
   l.total_tiles = (uint32_t)tiles;
   l.total_bins = (uint32_t)bins;
   l.bin_passes = bin_sort_passes(l.total_bins);
@@ -283,7 +294,7 @@ void Pipeline::ensure_workspace(const Layout &l) {
                                     kMaxSortItems)
                               : splat_cap_;
     // view workspace: [view counters | K1 status | emit status] zeroed, then the table.
-    const uint64_t k1_words = (ncap + 255) / 256 + 1;  // + views: blocks round up per set
+    const uint64_t k1_words = key_blocks(ncap) + 1;  // + views: blocks round up per set
     const uint64_t k1_total = k1_words + vcap;
     const uint64_t emit_words = emit_status_words(ncap);
     uint64_t off = 0;
@@ -437,15 +448,23 @@ void Pipeline::launch_all(const Layout &l, uint32_t *images, const HostSinks &si
   K1Buffers k1{vis_keys0_, vis_vals0_, rects_,         records_,
                k1_status_, counters_,  key_hist_,      view_counters_,
                debug_ ? projected_.as<ProjectedDev>() : nullptr, reuse};
+  // The depth sort needs the keys alone: it runs on the side stream, beside
+  // the vertex stage, and ahead of it where both want an SM (its passes are few
+  // blocks that wait for one another, the vertex stage many that do not).
+  launch_keys(views_dev, sets_dev, l.sets, l.key_blocks, k1, stream_);
+  if (!reuse) {  // a reused order keeps the last sort's ids and plan
+    GSR_CUDA(cudaEventRecord(fork_ev_, stream_));
+    GSR_CUDA(cudaStreamWaitEvent(side_stream_, fork_ev_, 0));
+    SortBuffers ds{vis_keys0_, vis_vals0_, vis_keys1_, vis_vals1_, &counters_->visible, n, 0, 4,
+                   depth_plan_, depth_sort_work_, &counters_->error, key_hist_, true};
+    ds.priority = side_priority_;
+    launch_sort(ds, side_stream_);
+    GSR_CUDA(cudaEventRecord(join_ev_, side_stream_));
+  }
   launch_preprocess(views_dev, sets_dev, l.sets, l.total_blocks, l.max_planes, k1, debug_,
                     stream_);
   record(1);
-
-  if (!reuse) {  // a reused order keeps the last sort's ids and plan
-    SortBuffers ds{vis_keys0_, vis_vals0_, vis_keys1_, vis_vals1_, &counters_->visible, n, 0, 4,
-                   depth_plan_, depth_sort_work_, &counters_->error, key_hist_, true};
-    launch_sort(ds, stream_);
-  }
+  if (!reuse) GSR_CUDA(cudaStreamWaitEvent(stream_, join_ev_, 0));
   record(2);
 
   EmitBuffers eb{depth_plan_, vis_vals0_,  vis_vals1_, rects_,        records_,
@@ -571,7 +590,7 @@ void Pipeline::enqueue(const ViewSpec *views, uint32_t count, uint32_t *images,
       capturing_ = false;
       GSR_CUDA(cudaStreamEndCapture(stream_, &g));
       cudaGraphExec_t exec = nullptr;
-      cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
+      cudaError_t e = cudaGraphInstantiate(&exec, g, cudaGraphInstantiateFlagUseNodePriority);
       if (e != cudaSuccess) {
         cudaGraphDestroy(g);
         throw Error(Code::Internal, std::string("CUDA graph instantiation failed: ") +
@@ -738,7 +757,7 @@ void Pipeline::enqueue_groups(const ViewSpec *views, uint32_t *images,
         capturing_ = false;
         GSR_CUDA(cudaStreamEndCapture(stream_, &g));
         cudaGraphExec_t exec = nullptr;
-        const cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
+        const cudaError_t e = cudaGraphInstantiate(&exec, g, cudaGraphInstantiateFlagUseNodePriority);
         if (e != cudaSuccess) {
           cudaGraphDestroy(g);
           throw Error(Code::Internal, std::string("CUDA graph instantiation failed: ") +
@@ -849,10 +868,10 @@ RunResult Pipeline::sync() {
 }
 
 uint32_t Pipeline::launches_per_run() const {
-  // preprocess; depth sort plan + 4 passes (histograms come from K1); emit;
-  // bin sort plan + passes (histograms from K2); ranges; raster.
+  // keys; preprocess; depth sort plan + 4 passes (histograms come from the
+  // keys); emit; bin sort plan + passes (histograms from K2); ranges; raster.
   const uint32_t bin_passes = last_layout_.bin_passes;
-  return 1 + (1 + 4) + 1 + (1 + bin_passes) + 1 + 1;
+  return 2 + (1 + 4) + 1 + (1 + bin_passes) + 1 + 1;
 }
 
 SortPlan Pipeline::read_plan(int which) {

@@ -185,12 +185,11 @@ class Pipeline {
 
  private:
   struct Layout {
-    uint32_t views = 0, total_splats = 0, total_blocks = 0, total_tiles = 0, total_bins = 0,
-             max_planes = 1;
+    uint32_t views = 0, total_splats = 0, total_blocks = 0, key_blocks = 0, total_tiles = 0, total_bins = 0, max_planes = 1;
     uint32_t bin_passes = 1, sets = 0;
     bool operator==(const Layout &o) const {
       return views == o.views && sets == o.sets && total_splats == o.total_splats &&
-             total_blocks == o.total_blocks && total_tiles == o.total_tiles &&
+             total_blocks == o.total_blocks && key_blocks == o.key_blocks && total_tiles == o.total_tiles &&
              total_bins == o.total_bins &&
              max_planes == o.max_planes && bin_passes == o.bin_passes;
     }
@@ -241,6 +240,9 @@ class Pipeline {
 
   int device_;
   cudaStream_t stream_;
+  cudaStream_t side_stream_ = nullptr;  // the depth sort; joined into stream_ within every run
+  int side_priority_ = 0;               // its priority, the highest
+  cudaEvent_t fork_ev_ = nullptr, join_ev_ = nullptr;
   cudaEvent_t ev_[kPhaseCount + 1] = {};
   uint32_t tile_ = 16, blend_mode_ = 0, sm_count_ = 148;
   RasterConfig raster_cfg_;
