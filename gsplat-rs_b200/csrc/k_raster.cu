@@ -24,6 +24,7 @@
 //     after every splat (the reference's Rgba8Unorm premultiplied blend).
 
 #include <algorithm>
+#include <type_traits>
 
 #include "bins.cuh"
 #include "device_common.cuh"
@@ -36,21 +37,16 @@
 #ifndef GSR_RASTER_F32X2
 #define GSR_RASTER_F32X2 1
 #endif
-// Resident blocks per SM the two-pixel FP32 kernel is compiled for: 8
-// blocks of 4 warps fit 64 registers a thread; 6 or 7 without spills run
-// slower (1.70 M pairs at 1920x1080: 122.9 and 118.8 us against 114.8), and
-// so do 10 or 12, which spill (122.8, 122.9).
-#ifndef GSR_RASTER_MIN_BLOCKS
-#define GSR_RASTER_MIN_BLOCKS 8
-#endif
-
-
 namespace gsr {
 namespace {
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
   uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
+  uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
@@ -187,8 +183,9 @@ __device__ __forceinline__ uint32_t nth_bit(uint32_t word, uint32_t n) {
 // positions), one per lane, and scans their bit counts; a thread then finds
 // the word and the bit of its own slots. No warp waits for another: a version
 // that split the words over the warps took two block barriers a step.
-template <int kThreads, int kChunk>
+template <int kThreads, int kChunk, bool kFromEnd>
 struct BinScan {
+  struct Smem {};
   uint32_t in_bin;      // the tile within its bin; bit 31: the sort's result is in buffer 0
   uint32_t begin, end;  // the list positions left
 
@@ -203,11 +200,13 @@ struct BinScan {
     end = range.y;
   }
 
-  // Starts the gather of the chunk's records into raw (16-byte async copies,
+  __device__ __forceinline__ void prime(const RasterArgs &, Smem &) {}
+
+  // Starts the gather of the next chunk's records into raw (16-byte async copies,
   // entry s in slot s) and calls each(gid, record) for them; returns their
   // number (0: the list is done). Every thread of the block calls it.
-  template <bool kFromEnd, typename F>
-  __device__ __forceinline__ uint32_t fill(const RasterArgs &a, float4 (&raw)[3][kChunk],
+  template <typename F>
+  __device__ __forceinline__ uint32_t next(const RasterArgs &a, Smem &, float4 (&raw)[3][kChunk],
                                            F each) {
     const uint32_t lane = threadIdx.x & 31;
     uint32_t filled = 0;
@@ -276,6 +275,181 @@ struct BinScan {
   }
 };
 
+// The same walk with its chain of loads, words -> ids -> records, spread over
+// three chunks: locate() starts the copies of the ids of the chunk after next
+// and of the words behind them, next() those of the records whose ids have
+// arrived. A window is 128 words, four to a lane. It costs more instructions
+// than BinScan and gathers ids that an early end does not need, so it pays
+// where a tile's own latency sets the time and not the throughput of many
+// (2 M splats on 475 tiles 72 -> 55 us at equal registers; 186 M pairs at 3840x2160
+// 397 -> 463).
+template <int kThreads, int kChunk, bool kFromEnd>
+struct BinScanAhead {
+  static constexpr uint32_t kNone = 0x80000000u;  // no window has this number
+  struct Smem {
+    uint4 window[4][32];  // window W's words in slot W % 4
+    uint32_t ids[kChunk];
+  };
+  uint32_t in_bin;      // the tile within its bin; bit 31: the sort's result is in buffer 0
+  uint32_t begin, end;  // the list
+  uint32_t window;      // the next entry's window, kNone when the list is done
+  uint32_t used;        // entries of the window already taken
+  uint32_t staged;      // this window and the next are in shared memory, or kNone
+  uint32_t located;     // entries of the next chunk
+
+  // (tx, ty): the tile within its view
+  __device__ __forceinline__ BinScanAhead(const RasterArgs &a, uint32_t bin_base, uint32_t tx,
+                                          uint32_t ty, uint32_t tiles_x) {
+    const uint32_t bin = bin_base + (ty / kBinEdge) * bins_along(tiles_x) + tx / kBinEdge;
+    const uint2 range = a.ranges[bin];
+    in_bin = (ty % kBinEdge) * kBinEdge + tx % kBinEdge;
+    if (a.plan->final_buffer == 0) in_bin |= 1u << 31;
+    begin = range.x;
+    end = range.y;
+    used = 0;
+    window = begin < end ? (kFromEnd ? end - 1 : begin) >> 12 : kNone;
+    staged = kNone;
+  }
+
+  __device__ __forceinline__ const uint4 *words(const RasterArgs &a, uint32_t w) const {
+    return reinterpret_cast<const uint4 *>(
+        &(in_bin >> 31 ? a.keys1 : a.keys0)[tile_word(w, in_bin & 15u)]);
+  }
+  // Whether any of the positions of words w .. w + 3 is in the list.
+  __device__ __forceinline__ bool in_list(uint32_t w) const {
+    return w >= (begin >> 7 << 2) && 32 * w < end;
+  }
+
+  // Starts the copies of the next chunk's ids (slot s's by the thread that
+  // gathers it) and returns their number (0: the list is done). Every thread
+  // of the block calls it, with a block barrier between two calls.
+  __device__ __forceinline__ uint32_t locate(const RasterArgs &a, Smem &sm) {
+    if (window == kNone) return 0;
+    const uint32_t lane = threadIdx.x & 31, quad = kFromEnd ? 31 - lane : lane;
+    const uint32_t was = staged;
+    uint32_t filled = 0;
+    while (filled < (uint32_t)kChunk && window != kNone) {
+      const uint32_t w = 128 * window + 4 * quad;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (in_list(w)) {
+        const uint32_t ahead = kFromEnd ? was - window : window - was;
+        v = was != kNone && ahead < 2 ? sm.window[window & 3][quad] : __ldg(words(a, w));
+      }
+      uint32_t bits[4] = {v.x, v.y, v.z, v.w};
+      if (4096 * window < begin || end - 4096 * window < 4096) {  // an end of the list
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+          const uint32_t p = 32 * (w + q);
+          if (p < begin) bits[q] &= begin - p >= 32 ? 0u : ~0u << (begin - p);
+          if (p >= end) bits[q] = 0u;
+          else if (end - p < 32) bits[q] &= (1u << (end - p)) - 1u;
+        }
+      }
+      if (kFromEnd) {  // bit i of word q: position 32 (w + 3 - q) + 31 - i
+        const uint32_t b0 = __brev(bits[0]), b1 = __brev(bits[1]);
+        bits[0] = __brev(bits[3]), bits[1] = __brev(bits[2]);
+        bits[2] = b1, bits[3] = b0;
+      }
+      // counts of the words before words 1, 2, 3 and of all four, one per byte
+      uint32_t pre = __popc(bits[0]);
+      pre |= (pre + __popc(bits[1])) << 8;
+      pre |= ((pre >> 8) + __popc(bits[2])) << 16;
+      pre |= ((pre >> 16) + __popc(bits[3])) << 24;
+      uint32_t inc = pre >> 24;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += t;
+      }
+      const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
+      const uint32_t taken = min(total - used, (uint32_t)kChunk - filled);
+#pragma unroll
+      for (uint32_t t0 = 0; t0 < (uint32_t)kChunk; t0 += kThreads) {
+        // this thread's slot, if the window fills any of the warp's
+        const uint32_t slot = t0 + threadIdx.x;
+        const bool in = slot >= filled && slot - filled < taken;
+        if (!__any_sync(0xffffffffu, in)) continue;
+        const uint32_t n = in ? slot - filled + used : 0u;
+        uint32_t c = 0;  // the first lane whose inclusive count exceeds n
+#pragma unroll
+        for (uint32_t step = 16; step >= 1; step >>= 1)
+          if (__shfl_sync(0xffffffffu, inc, c + step - 1) <= n) c += step;
+        const uint32_t cp = __shfl_sync(0xffffffffu, pre, c);
+        uint32_t r = n + (cp >> 24) - __shfl_sync(0xffffffffu, inc, c);
+        uint32_t word = __shfl_sync(0xffffffffu, bits[0], c);
+        uint32_t q = 0, before = 0;
+#pragma unroll
+        for (uint32_t k = 1; k < 4; ++k) {
+          const uint32_t wk = __shfl_sync(0xffffffffu, bits[k], c);
+          const uint32_t pk = (cp >> (8 * (k - 1))) & 255u;
+          if (r >= pk) q = k, word = wk, before = pk;
+        }
+        if (in) {
+          const uint32_t at = 32 * q + nth_bit(word, r - before);
+          const uint32_t pos =
+              4096 * window + (kFromEnd ? 4095 - (128 * c + at) : 128 * c + at);
+          cp_async4(&sm.ids[slot], &(in_bin >> 31 ? a.ids0 : a.ids1)[pos]);
+        }
+      }
+      filled += taken;
+      used += taken;
+      if (used == total) {
+        used = 0;
+        const bool last = kFromEnd ? window == begin >> 12 : window == (end - 1) >> 12;
+        window = last ? kNone : kFromEnd ? window - 1 : window + 1;
+      }
+    }
+    // The cursor's window and the one behind it go to shared memory for the
+    // next call. Other warps may still read the two that were there: two
+    // windows further at most, the four slots keep them apart.
+    if (window != kNone) {
+      const uint32_t ahead = kFromEnd ? was - window : window - was;
+      if (was != kNone && ahead > 2) {
+        staged = kNone;
+      } else {
+        staged = window;
+        const uint32_t have = was == kNone || ahead == 2 ? 0 : 2 - ahead;
+        if (threadIdx.x < 32)
+          for (uint32_t k = have; k < 2; ++k) {
+            const uint32_t win = kFromEnd ? window - k : window + k;
+            const uint32_t w = 128 * win + 4 * lane;
+            if (win < kNone && in_list(w)) cp_async16(&sm.window[win & 3][lane], words(a, w));
+          }
+      }
+    }
+    return filled;
+  }
+
+  // The first chunk's ids, which the first next() gathers by.
+  __device__ __forceinline__ void prime(const RasterArgs &a, Smem &sm) {
+    located = locate(a, sm);
+    cp_async_wait_all();
+    __syncthreads();
+  }
+
+  // As BinScan's. Between two calls every thread waits for its copies and
+  // then for the block.
+  template <typename F>
+  __device__ __forceinline__ uint32_t next(const RasterArgs &a, Smem &sm,
+                                           float4 (&raw)[3][kChunk], F each) {
+    const uint32_t n = located;
+#pragma unroll
+    for (uint32_t t0 = 0; t0 < (uint32_t)kChunk; t0 += kThreads) {
+      const uint32_t slot = t0 + threadIdx.x;
+      if (slot < n) {
+        const uint32_t gid = sm.ids[slot];
+        const Record *r = &a.records[gid];
+        cp_async16(&raw[0][slot], &r->a);
+        cp_async16(&raw[1][slot], &r->b);
+        cp_async16(&raw[2][slot], &r->c);
+        each(gid, r);
+      }
+    }
+    located = locate(a, sm);
+    return n;
+  }
+};
+
 // UNORM8 parity mode: back to front over the tile list (forwards), the
 // reference fragment rule with the quad clip, and the premultiplied OVER
 // blend rounded to UNORM8 after every splat, exactly as the oracle's
@@ -288,13 +462,16 @@ struct BinScan {
 // 1e-6: alpha e^(-4.5 r^2) > 1/256 holds only below s^2 up to rounding), and
 // each warp walks only the entries whose mask has its bit. A channel keeps
 // its stored byte t as f = RN(t / 255), the float the next blend reads.
-template <int kTile>
+template <int kTile, bool kAhead>
 struct U8Smem {
   static constexpr int kThreads = kTile * kTile;
   static constexpr int kWarps = kThreads / 32;
-  static constexpr int kChunk = kTile * kTile;
+  static constexpr int kChunk = kTile == 16 || kAhead ? 256 : 128;
+  using Scan = std::conditional_t<kAhead, BinScanAhead<kThreads, kChunk, false>,
+                                  BinScan<kThreads, kChunk, false>>;
   float4 raw[2][3][kChunk];  // (cx, cy, ax, ay), (bx, by, s, alpha), premultiplied rgb
-  uint32_t list[kWarps][kChunk];
+  typename Scan::Smem scan;
+  alignas(16) uint32_t list[kWarps][kChunk];  // read by pairs
   uint32_t bits[kWarps][kChunk / 32];
   uint32_t view;
 };
@@ -334,11 +511,18 @@ __device__ __forceinline__ float2 unorm8_step(float2 f, float om, float2 src) {
 }
 
 // 16x16 tiles: compiled for 4 resident blocks per SM (up to 64 registers a
-// thread), which measured 2% faster than 5 blocks at 48 registers.
-template <int kTile>
-__global__ void __launch_bounds__(kTile *kTile, kTile == 16 ? 4 : 1)
+// thread), which measured 2% faster than 5 blocks at 48 registers; weights of
+// two entries are in flight a step (four at 3 or 2 blocks: 514 -> 516 us,
+// 1920x1080 with 1.70 M pairs). 8x8 tiles keep four in flight at 12 blocks
+// (279 k splats at 1280x720: 349 -> 317 us). kAhead: few tiles (up to 4 of
+// 16x16 a SM), where the tile with the longest list sets the time and a warp of it is
+// bound by its own chain of latencies: four entries in flight at half the
+// blocks, chunks of 256 and a list walked ahead (144 tiles of 187 k splats
+// 670 -> 594 us, 608 tiles of 8x8 and 258 k splats 807 -> 583).
+template <int kTile, bool kAhead>
+__global__ void __launch_bounds__(kTile *kTile, kTile == 16 ? (kAhead ? 2 : 4) : (kAhead ? 8 : 12))
     raster_unorm8_kernel(RasterArgs a) {
-  using Smem = U8Smem<kTile>;
+  using Smem = U8Smem<kTile, kAhead>;
   constexpr int kN = Smem::kChunk;
   constexpr int kThreads = Smem::kThreads;
   constexpr int kBlocksX = kTile / 8;
@@ -358,9 +542,9 @@ __global__ void __launch_bounds__(kTile *kTile, kTile == 16 ? 4 : 1)
   const bool inside = px < width && py < height;
   const float fpx = (float)px, fpy = (float)py;
   const float ftx = (float)x0, fty = (float)y0;
-  BinScan<kThreads, kN> scan(a, a.views[view].bin_base, tx, ty, tiles_x);
+  typename Smem::Scan scan(a, a.views[view].bin_base, tx, ty, tiles_x);
   auto fill = [&](int buf) {
-    return scan.template fill<false>(a, sm.raw[buf], [](uint32_t, const Record *) {});
+    return scan.next(a, sm.scan, sm.raw[buf], [](uint32_t, const Record *) {});
   };
   // j is the entry's byte offset in raw, its first float4
   auto at = [&](uint32_t j, uint32_t q) {
@@ -392,6 +576,7 @@ __global__ void __launch_bounds__(kTile *kTile, kTile == 16 ? 4 : 1)
     rg = unorm8_step(rg, om, mul2(make_float2(pc.x, pc.y), pair(g)));
     ba = unorm8_step(ba, om, make_float2(__fmul_rn(pc.z, g), w));
   };
+  scan.prime(a, sm.scan);
   uint32_t n_in = fill(0);
   for (int buf = 0; n_in; buf ^= 1) {
     // every thread's records have landed, and the chunk before is blended
@@ -415,20 +600,31 @@ __global__ void __launch_bounds__(kTile *kTile, kTile == 16 ? 4 : 1)
     const uint32_t n_w = list_entries(sm.bits[warp], buf * (uint32_t)sizeof(sm.raw[0]), list);
     if (inside) {
       uint32_t i = 0;
-      // two entries per step: the second's coverage and weight do not wait
-      // for the first's blend
-      for (; i + 1 < n_w; i += 2) {
-        const uint2 jj = *reinterpret_cast<const uint2 *>(&list[i]);
-        float ga, wa, gb, wb;
-        weight(jj.x, ga, wa);
-        weight(jj.y, gb, wb);
-        blend(jj.x, ga, wa);
-        blend(jj.y, gb, wb);
+      // several entries per step: the later ones' coverage and weight do not
+      // wait for the first's blend
+      constexpr int kStep = kAhead || kTile == 8 ? 4 : 2;
+      for (; i + (kStep - 1) < n_w; i += kStep) {
+        uint32_t jj[kStep];
+        float g[kStep], w[kStep];
+#pragma unroll
+        for (int k = 0; k < kStep; k += 2) {
+          const uint2 two = *reinterpret_cast<const uint2 *>(&list[i + k]);
+          jj[k] = two.x, jj[k + 1] = two.y;
+        }
+#pragma unroll
+        for (int k = 0; k < kStep; ++k) weight(jj[k], g[k], w[k]);
+#pragma unroll
+        for (int k = 0; k < kStep; ++k) blend(jj[k], g[k], w[k]);
       }
-      if (i < n_w) {
+      auto one = [&]() {
         float g, w;
         weight(list[i], g, w);
         blend(list[i], g, w);
+      };
+      if constexpr (kStep == 2) {
+        if (i < n_w) one();
+      } else {
+        for (; i < n_w; ++i) one();
       }
     }
     n_in = n_next;
@@ -438,6 +634,15 @@ __global__ void __launch_bounds__(kTile *kTile, kTile == 16 ? 4 : 1)
     image[(size_t)py * width + px] = to_unorm8(rg.x) | (to_unorm8(rg.y) << 8) |
                                      (to_unorm8(ba.x) << 16) | (to_unorm8(ba.y) << 24);
 }
+
+// Resident blocks per SM the FP32 kernel is compiled for with more tiles than
+// are resident: 8 blocks of 4 warps fit 64 registers a thread; 6 or 7 without
+// spills run slower (1.70 M pairs at 1920x1080: 122.9 and 118.8 us against
+// 114.8), and so do 10 or 12, which spill (122.8, 122.9). 8x8 tiles: 16
+// blocks of 2 warps (279 k splats at 1280x720: 111 us with the 9 that 97
+// registers allow, 92 here).
+template <int kTile>
+constexpr int kManyBlocks = kTile == 16 ? 8 : 16;
 
 // FP32 front-to-back mode. kPx = 1: threads map to 8x4-pixel warp blocks
 // (lane l of warp w covers column (w % (kTile/8))*8 + (l & 7), row
@@ -462,7 +667,7 @@ __global__ void __launch_bounds__(kTile *kTile, kTile == 16 ? 4 : 1)
 // Culling is conservative, so results equal the unculled per-pixel walk, and
 // neither the chunk size, the pixels per thread nor the tile order changes
 // any pixel.
-template <int kTile, int kChunk, int kPx>
+template <int kTile, int kChunk, int kPx, bool kAhead>
 struct Fp32Smem {
   static_assert(kPx == 1 || (kPx == 2 && kTile == 16), "two pixels per thread on 16x16 tiles");
   static constexpr int kThreads = kTile * kTile / kPx;
@@ -470,18 +675,22 @@ struct Fp32Smem {
   // Chunk records as they arrive (a, b, c), overwritten in place by the
   // per-tile entry data: [0] = ax, ay, ox, thr (coverage bound on r^2);
   // [1] = bx, by, oy, -; [2] = r, g, b, log2 alpha (the record's c).
+  using Scan = std::conditional_t<kAhead, BinScanAhead<kThreads, kChunk, true>,
+                                  BinScan<kThreads, kChunk, true>>;
   float4 raw[2][3][kChunk];
+  typename Scan::Smem scan;
   alignas(16) uint32_t list[kWarps][kChunk];
   uint32_t bits[kWarps][kChunk / 32];
   uint32_t view;
   uint32_t next;
 };
 
-template <int kTile, int kChunk, int kPx>
+template <int kTile, int kChunk, int kPx, bool kAhead>
 __device__ __forceinline__ void raster_fp32_tile(const RasterArgs &a, uint32_t tile,
-                                                 Fp32Smem<kTile, kChunk, kPx> &sm) {
+                                                 Fp32Smem<kTile, kChunk, kPx, kAhead> &sm) {
   constexpr int kBlocksX = kTile / 8;
-  constexpr int kThreads = Fp32Smem<kTile, kChunk, kPx>::kThreads;
+  using Smem = Fp32Smem<kTile, kChunk, kPx, kAhead>;
+  constexpr int kThreads = Smem::kThreads;
   constexpr int kRows = 4 * kPx;  // rows of a warp's block
   const uint32_t view = block_view(a, tile, sm.view);
   const uint32_t width = a.views[view].p.width, height = a.views[view].p.height;
@@ -508,9 +717,9 @@ __device__ __forceinline__ void raster_fp32_tile(const RasterArgs &a, uint32_t t
   }
   const float fax = (float)ax0, fay = (float)ay0;
   const float ftx = (float)x0, fty = (float)y0;
-  BinScan<kThreads, kChunk> scan(a, a.views[view].bin_base, tx, ty, tiles_x);
+  typename Smem::Scan scan(a, a.views[view].bin_base, tx, ty, tiles_x);
   auto fill = [&](int buf) {
-    return scan.template fill<true>(a, sm.raw[buf], [&](uint32_t gid, const Record *r) {
+    return scan.next(a, sm.scan, sm.raw[buf], [&](uint32_t gid, const Record *r) {
       // debug tap: the inputs and the bound this kernel blends with (every
       // tile of a splat writes the same pair)
       if (a.debug_cov) {
@@ -534,6 +743,7 @@ __device__ __forceinline__ void raster_fp32_tile(const RasterArgs &a, uint32_t t
     for (int p = 0; p < kPx; ++p) d = d && done[p];
     return d;
   };
+  scan.prime(a, sm.scan);
   uint32_t n_in = fill(0);
   cp_async_wait_all();
   __syncthreads();
@@ -664,20 +874,21 @@ __device__ __forceinline__ void raster_fp32_tile(const RasterArgs &a, uint32_t t
 // One block per tile (kPersistent false), or a fixed grid of blocks that take
 // tiles from a global queue (an atomic ticket over the batch's tiles) until
 // it is empty.
-template <int kTile, int kChunk, int kPx, bool kPersistent>
-__global__ void __launch_bounds__(kTile *kTile / kPx, kPx == 2 ? GSR_RASTER_MIN_BLOCKS : 1)
+template <int kTile, int kChunk, int kPx, int kBlocks, bool kPersistent>
+__global__ void __launch_bounds__(kTile *kTile / kPx, kBlocks)
     raster_fp32_kernel(RasterArgs a) {
-  __shared__ Fp32Smem<kTile, kChunk, kPx> sm;
+  constexpr bool kAhead = kBlocks < kManyBlocks<kTile>;
+  __shared__ Fp32Smem<kTile, kChunk, kPx, kAhead> sm;
   fold_errors(a);
   if constexpr (!kPersistent) {
-    raster_fp32_tile<kTile, kChunk, kPx>(a, blockIdx.x, sm);
+    raster_fp32_tile<kTile, kChunk, kPx, kAhead>(a, blockIdx.x, sm);
   } else {
     for (;;) {
       if (threadIdx.x == 0) sm.next = atomicAdd(&a.counters->raster_ticket, 1u);
       __syncthreads();
       const uint32_t tile = sm.next;
       if (tile >= a.total_tiles) break;
-      raster_fp32_tile<kTile, kChunk, kPx>(a, tile, sm);
+      raster_fp32_tile<kTile, kChunk, kPx, kAhead>(a, tile, sm);
       __syncthreads();  // shared memory is reused by the next tile
     }
   }
@@ -689,36 +900,50 @@ void launch_raster(const RasterArgs &a, uint32_t tile, uint32_t blend_mode,
                    const RasterConfig &cfg, uint32_t sm_count, cudaStream_t stream) {
   if (a.total_tiles == 0) return;
   if (blend_mode == 1) {
-    if (tile == 16)
-      raster_unorm8_kernel<16><<<a.total_tiles, 256, 0, stream>>>(a);
-    else
-      raster_unorm8_kernel<8><<<a.total_tiles, 64, 0, stream>>>(a);
+    // At most 4 tiles a SM (16 of 8x8 pixels): see raster_unorm8_kernel.
+    const bool ahead = a.total_tiles <= (tile == 16 ? 4 : 16) * sm_count;
+#define GSR_U8(T, A) raster_unorm8_kernel<T, A><<<a.total_tiles, T * T, 0, stream>>>(a)
+    if (tile == 16) {
+      if (ahead) GSR_U8(16, true);
+      else GSR_U8(16, false);
+    } else {
+      if (ahead) GSR_U8(8, true);
+      else GSR_U8(8, false);
+    }
+#undef GSR_U8
     return;
   }
   const bool persistent = cfg.blocks_per_sm > 0;
   const uint32_t grid =
       persistent ? std::min<uint32_t>(a.total_tiles, cfg.blocks_per_sm * sm_count) : a.total_tiles;
-#define GSR_FP32(T, C, P)                                                        \
+  const uint32_t per_sm = (a.total_tiles + sm_count - 1) / sm_count;
+#define GSR_FP32(T, C, P, B)                                                     \
   do {                                                                           \
     if (persistent)                                                              \
-      raster_fp32_kernel<T, C, P, true><<<grid, T * T / P, 0, stream>>>(a);      \
+      raster_fp32_kernel<T, C, P, B, true><<<grid, T * T / P, 0, stream>>>(a);   \
     else                                                                         \
-      raster_fp32_kernel<T, C, P, false><<<grid, T * T / P, 0, stream>>>(a);     \
+      raster_fp32_kernel<T, C, P, B, false><<<grid, T * T / P, 0, stream>>>(a);  \
   } while (0)
+  // With few tiles the one with the longest list sets the time, and a warp of
+  // it is bound by its own latencies: the registers that no further block
+  // would use go to it (4 or 7 blocks a SM instead of 8, 8 of 8x8 tiles
+  // instead of 16), its list is walked ahead, and the steps are longer (us, 8
+  // blocks and a direct walk -> as here: 256 tiles of 27 k pairs 32.8 -> 28.7,
+  // 190 tiles, 62 k splats 110.6 -> 84.0, 475 tiles, 2 M splats 71.7 -> 49.2;
+  // 750 tiles of 100 k splats 59.4 -> 55.3 at 7 blocks). A chunk is the most a
+  // step stages: with more tiles than blocks are resident half of 256 is
+  // better, since a tile that fills up early has then gathered fewer records
+  // it does not need and 8 blocks fit (1.70 M pairs at 1920x1080 116.9 ->
+  // 112.6 us, 186 M at 3840x2160 500 -> 397).
   if (tile == 16) {
-    // A chunk of 256 is the most a step stages: with more tiles than blocks
-    // of it are resident (7 per SM) half as much is, since a tile that fills
-    // up early has then gathered fewer records it does not need and 8 blocks
-    // fit (1.70 M pairs at 1920x1080 116.9 -> 112.6 us, 186 M at 3840x2160
-    // 500 -> 397); with all tiles resident fewer, larger steps are faster
-    // (256 tiles: 33.8 -> 32.8 us).
-    const bool resident = a.total_tiles <= 7 * sm_count;
-    if (cfg.chunk == 64) GSR_FP32(16, 64, GSR_RASTER_PX);
-    else if (cfg.chunk == 128 || !resident) GSR_FP32(16, 128, GSR_RASTER_PX);
-    else GSR_FP32(16, 256, GSR_RASTER_PX);
+    if (cfg.chunk == 64) GSR_FP32(16, 64, GSR_RASTER_PX, kManyBlocks<16>);
+    else if (cfg.chunk == 128 || per_sm > 7) GSR_FP32(16, 128, GSR_RASTER_PX, kManyBlocks<16>);
+    else if (per_sm > 4) GSR_FP32(16, 256, GSR_RASTER_PX, 7);
+    else GSR_FP32(16, 256, GSR_RASTER_PX, 4);
   } else {
-    if (cfg.chunk == 32) GSR_FP32(8, 32, 1);
-    else GSR_FP32(8, 64, 1);
+    if (cfg.chunk == 32) GSR_FP32(8, 32, 1, kManyBlocks<8>);
+    else if (per_sm > 16) GSR_FP32(8, 64, 1, kManyBlocks<8>);
+    else GSR_FP32(8, 128, 1, 8);
   }
 #undef GSR_FP32
 }
