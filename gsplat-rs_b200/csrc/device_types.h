@@ -73,7 +73,12 @@ enum : uint32_t {
 
 // Per-frame device counters; zeroed before each frame.
 struct FrameCounters {
-  uint32_t k1_ticket;
+  // Starts of the phases in ns (global_ns()): the zeroing kernel's end, the
+  // vertex stage's last block for the remainder of the depth sort, then the
+  // first kernel of each; [6], in the host copies of frames alone, the raster's end. Not
+  // zeroed but set by the zeroing kernel.
+  unsigned long long phase_ns[7];
+  uint32_t k1_ticket;  // zeroed at the start of a run from here on
   uint32_t emit_ticket;
   uint32_t visible;
   uint32_t drawn;
@@ -83,6 +88,8 @@ struct FrameCounters {
   uint32_t raster_ticket;  // persistent raster tile queue
   unsigned long long keys;  // (tile, splat) pairs they stand for (may exceed the capacity)
   uint32_t sort_tickets[16];
+  uint32_t sticky;  // host copies alone: the sticky word as of this run
+  uint32_t raster_done;  // blocks of the raster that are done
 };
 
 // One view of a frame batch (a plain frame is a batch of one view). Splats

@@ -675,9 +675,12 @@ __global__ void __launch_bounds__(kK1Threads, GSR_K1_MIN_BLOCKS)
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0 && !s_lost) {  // every thread has passed both waits
-    mbar_inval(&st.bar[0]);
-    mbar_inval(&st.bar[1]);
+  if (threadIdx.x == 0) {
+    atomicMax(&b.counters->phase_ns[1], global_ns());
+    if (!s_lost) {  // every thread has passed both waits
+      mbar_inval(&st.bar[0]);
+      mbar_inval(&st.bar[1]);
+    }
   }
 }
 

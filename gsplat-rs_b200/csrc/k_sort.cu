@@ -102,7 +102,9 @@ __global__ void __launch_bounds__(kThreads) plan_kernel(const uint32_t *__restri
                                                         const uint32_t *__restrict__ hist,
                                                         uint32_t passes, SortPlan *plan,
                                                         uint32_t *status, uint32_t tile_stride,
-                                                        uint32_t tile_items) {
+                                                        uint32_t tile_items,
+                                                        unsigned long long *start_ns) {
+  if (start_ns && blockIdx.x == 0 && threadIdx.x == 0) *start_ns = global_ns();
   constexpr uint32_t kDigits = kThreads * kDpt;
   const uint32_t n = *count;
   const uint64_t used = (uint64_t)((n + tile_items - 1) / tile_items) * kDigits;  // words per pass
@@ -657,7 +659,7 @@ void launch_wide(const SortBuffers &b, cudaStream_t stream) {
   uint32_t *status = b.work + kSortScratchHeadWords;
   launch_at(b, plan_kernel<(1 << kBits) / kThreads>,
             std::min<uint32_t>(tiles, 2 * device_sm_count()), stream, b.count, b.hist, 1, b.plan,
-            status, tiles, kTile);
+            status, tiles, kTile, b.start_ns);
   const uint32_t grid = std::min(tiles, resident_blocks<wide_kernel<kBits>>());
   launch_at(b, wide_kernel<kBits>, grid, stream, b.plan, b.begin_bit, b.keys0, b.vals0, b.keys1,
             b.vals1, status, b.work, b.error);
@@ -685,7 +687,7 @@ void launch_sort(const SortBuffers &b, cudaStream_t stream) {
   }
   const uint32_t zero_blocks = std::min<uint32_t>(grid, 2 * device_sm_count());
   launch_at(b, plan_kernel<1>, zero_blocks, stream, b.count, b.hist ? b.hist : hist, b.passes,
-            b.plan, status, tiles, kThreads * ipt);
+            b.plan, status, tiles, kThreads * ipt, b.start_ns);
   constexpr int kSmall = GSR_SORT_MIN_BLOCKS, kLarge = GSR_SORT_MIN_BLOCKS_LARGE;
   for (uint32_t p = 0; p < b.passes; ++p) {
     auto pass = [&](auto kernel, uint32_t resident) {

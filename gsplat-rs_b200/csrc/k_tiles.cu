@@ -144,6 +144,7 @@ __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EmitBuffers b) {
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t hist_words = b.wide_bits ? 1u << b.wide_bits : b.bin_passes * 256;
   const uint32_t low_mask = b.wide_bits ? hist_words - 1u : 255u;
+  if (blockIdx.x == 0 && tid == 0) b.counters->phase_ns[2] = global_ns();
   for (uint32_t k = tid; k < hist_words; k += kEmitThreads) s_hist[k] = 0;
   for (uint32_t v = tid; v < b.num_views; v += kEmitThreads) {
     s_vsb[v] = b.views[v].splat_base;
@@ -359,7 +360,10 @@ __global__ void __launch_bounds__(256) ranges_kernel(const SortPlan *__restrict_
   const bool first = plan->final_buffer == 0;
   const uint32_t *keys = first ? k0 : k1;
   uint32_t *words = first ? k1 : k0;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && counters->keys > capacity) counters->overflow = 1u;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    counters->phase_ns[4] = global_ns();
+    if (counters->keys > capacity) counters->overflow = 1u;
+  }
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * blockDim.x / 32, groups = (K + 255) / 256;
   for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / 32; g < groups; g += warps) {
@@ -426,6 +430,10 @@ __global__ void run_init_kernel(RunInit a) {
 #pragma unroll
   for (int r = 0; r < kRunZeroRegions; ++r)
     for (uint64_t i = t; i < a.zero_words[r]; i += stride) a.zero[r][i] = 0u;
+  if (t == 0) {
+    const unsigned long long now = global_ns();
+    for (int k = 0; k < 6; ++k) a.phase_ns[k] = now;
+  }
 }
 
 __global__ void fill_kernel(uint32_t *dst, uint32_t value, uint64_t count) {

@@ -72,6 +72,7 @@ struct SortBuffers {
   // sort_work_words of 4 passes).
   uint32_t wide_bits = 0;
   int priority = 0;  // launch priority of the kernels (as a stream's)
+  unsigned long long *start_ns = nullptr;  // when the sort starts, if wanted
 };
 constexpr uint32_t kSortScratchHeadWords = 64 + 4 * 256;  // tickets and histograms
 uint64_t sort_work_words(uint32_t capacity, uint32_t passes);
@@ -127,6 +128,11 @@ struct RasterArgs {
   uint32_t *images;
   FrameCounters *counters;         // raster_ticket is the persistent tile queue
   uint32_t *sticky;
+  const ViewCounters *view_counters;
+  // Host copies of the counters (pinned memory), which block 0 writes.
+  FrameCounters *host_counters;
+  ViewCounters *host_views;
+  unsigned long long *end_ns;      // pinned: when the raster ends, if wanted
   float2 *debug_cov = nullptr;     // debug tap: (log2 alpha, coverage bound) per splat slot
 };
 // Raster launch shape: records staged per step (tile 16: 64/128/256; tile 8:
@@ -158,6 +164,7 @@ constexpr uint32_t kRunInlineViews = 8;
 struct RunInit {
   uint32_t *zero[kRunZeroRegions];       // regions zeroed at the start of a run
   uint64_t zero_words[kRunZeroRegions];
+  unsigned long long *phase_ns;          // set to the end of this kernel
   uint32_t inline_views = 0;  // 0: the table was copied to the device beforehand
   uint32_t inline_sets = 0;
   ViewSetDev *sets_dst = nullptr;

@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cstddef>
 #include <cstring>
 #include <string>
 
@@ -134,7 +135,6 @@ Pipeline::Pipeline(int device, cudaStream_t stream) : device_(device), stream_(s
   int sms = 0;
   GSR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
   sm_count_ = (uint32_t)sms;
-  for (auto &ev : ev_) GSR_CUDA(cudaEventCreate(&ev));
   for (auto &ev : slot_ev_) GSR_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   int least = 0, greatest = 0;
   GSR_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
@@ -172,8 +172,6 @@ Pipeline::~Pipeline() {
   if (side_stream_) cudaStreamDestroy(side_stream_);
   if (fork_ev_) cudaEventDestroy(fork_ev_);
   if (join_ev_) cudaEventDestroy(join_ev_);
-  for (auto &ev : ev_)
-    if (ev) cudaEventDestroy(ev);
   for (auto &ev : slot_ev_)
     if (ev) cudaEventDestroy(ev);
 
@@ -182,14 +180,6 @@ Pipeline::~Pipeline() {
   if (table_pinned_) cudaFreeHost(table_pinned_);
   if (batch_stage_) cudaFreeHost(batch_stage_);
   if (batch_ev_) cudaEventDestroy(batch_ev_);
-}
-
-void Pipeline::record(int k) {
-  if (batch_mode_) return;  // a batch of groups is timed by its caller
-  if (capturing_)
-    GSR_CUDA(cudaEventRecordWithFlags(ev_[k], stream_, cudaEventRecordExternal));
-  else
-    GSR_CUDA(cudaEventRecord(ev_[k], stream_));
 }
 
 void Pipeline::set_tile(uint32_t tile) {
@@ -418,8 +408,10 @@ void Pipeline::ensure_key_workspace(uint64_t capacity) {
 
 RunInit Pipeline::make_run_init(const Layout &l) const {
   RunInit init{};
-  init.zero[0] = fixed_.as<uint32_t>();
-  init.zero_words[0] = ((char *)depth_plan_ - (char *)fixed_.get()) / 4;
+  constexpr size_t kKept = offsetof(FrameCounters, k1_ticket);
+  init.zero[0] = fixed_.as<uint32_t>(kKept);
+  init.zero_words[0] = ((char *)depth_plan_ - (char *)fixed_.get() - kKept) / 4;
+  init.phase_ns = counters_->phase_ns;
   init.zero[1] = view_ws_.as<uint32_t>();
   init.zero_words[1] = view_zero_bytes_ / 4;
   init.zero[2] = reinterpret_cast<uint32_t *>(ranges_);
@@ -443,7 +435,6 @@ void Pipeline::launch_all(const Layout &l, uint32_t *images, const HostSinks &si
                           bool reuse, const ViewDev *views_dev, const ViewSetDev *sets_dev) {
   const uint32_t n = std::max<uint32_t>(l.total_splats, 1);
   launch_run_init(make_run_init(l), stream_);
-  record(0);
 
   K1Buffers k1{vis_keys0_, vis_vals0_, rects_,         records_,
                k1_status_, counters_,  key_hist_,      view_counters_,
@@ -463,9 +454,7 @@ void Pipeline::launch_all(const Layout &l, uint32_t *images, const HostSinks &si
   }
   launch_preprocess(views_dev, sets_dev, l.sets, l.total_blocks, l.max_planes, k1, debug_,
                     stream_);
-  record(1);
   if (!reuse) GSR_CUDA(cudaStreamWaitEvent(stream_, join_ev_, 0));
-  record(2);
 
   EmitBuffers eb{depth_plan_, vis_vals0_,  vis_vals1_, rects_,        records_,
                  pair_keys0_, pair_vals0_, key_cap_,   emit_status_,  counters_,
@@ -478,35 +467,25 @@ void Pipeline::launch_all(const Layout &l, uint32_t *images, const HostSinks &si
     GSR_CUDA(cudaMemcpyAsync(debug_pairs_.as<uint32_t>(4 * key_cap_), pair_vals0_, 4 * key_cap_,
                              cudaMemcpyDeviceToDevice, stream_));
   }
-  record(3);
   SortBuffers ts{pair_keys0_, pair_vals0_, pair_keys1_, pair_vals1_, &counters_->pairs,
                  (uint32_t)key_cap_, kBinCodeBits, l.bin_passes, bin_plan_, pair_sort_work_,
                  &counters_->error, bin_hist_, true};
   ts.expected = std::max<uint32_t>((uint32_t)(key_cap_ / kPairsPerBinPair), 1);
   ts.wide_bits = bin_wide_bits(l.total_bins);
+  ts.start_ns = &counters_->phase_ns[kPhaseTileSort];
   launch_sort(ts, stream_);
-  record(4);
   launch_ranges(bin_plan_, pair_keys0_, pair_keys1_, counters_, (uint32_t)key_cap_, ranges_,
                 stream_);
-  record(5);
   RasterArgs ra{views_dev,  l.views,  l.total_tiles, ranges_,   bin_plan_,
                 pair_keys0_, pair_vals0_, pair_keys1_, pair_vals1_, records_, images, counters_,
-                sticky_};
+                sticky_,     view_counters_, sinks.counters, sinks.views,
+                batch_mode_ ? nullptr : &sinks.counters->phase_ns[kPhaseCount]};
   if (debug_) {
     GSR_CUDA(cudaMemsetAsync(debug_cov_.get(), 0xff, 8ull * std::max<uint32_t>(l.total_splats, 1),
                              stream_));
     ra.debug_cov = debug_cov_.as<float2>();
   }
   launch_raster(ra, tile_, blend_mode_, raster_cfg_, sm_count_, stream_);
-  record(6);
-  // Runs with host sinks copy their counters there; the others leave them in
-  // device memory, read after the stream is synchronised.
-  if (sinks.counters) {
-    GSR_CUDA(cudaMemcpyAsync(sinks.counters, counters_, sizeof(FrameCounters),
-                             cudaMemcpyDeviceToHost, stream_));
-    GSR_CUDA(cudaMemcpyAsync(sinks.views, view_counters_, sizeof(ViewCounters) * l.views,
-                             cudaMemcpyDeviceToHost, stream_));
-  }
 }
 
 void Pipeline::enqueue(const ViewSpec *views, uint32_t count, uint32_t *images,
@@ -514,10 +493,7 @@ void Pipeline::enqueue(const ViewSpec *views, uint32_t count, uint32_t *images,
   GSR_CUDA(cudaSetDevice(device_));
   const Layout l = plan_views(views, count, image_bases);
   ensure_workspace(l);
-  // No sinks given: the counters stay in device memory until the host reads
-  // them after a synchronisation (no host memory traffic inside the run).
-  const bool device_sinks = !sinks.counters;
-  if (device_sinks) sinks = HostSinks{};
+  if (!sinks.counters) sinks = HostSinks{counters_host_, view_counters_pinned_};
   // The last sorted order can be reused only for the identical layout (same
   // scenes, sizes and tile grid) and while its buffers are intact.
   const bool reuse = reuse_request_ && sorted_valid_ && l == sorted_layout_ &&
@@ -577,17 +553,14 @@ void Pipeline::enqueue(const ViewSpec *views, uint32_t count, uint32_t *images,
       cudaGraph_t g = nullptr;
       const auto t_capture = std::chrono::steady_clock::now();
       GSR_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-      capturing_ = true;
       try {
         launch_all(l, images, sinks, reuse, run_views, run_sets);
       } catch (...) {
-        capturing_ = false;
         cudaStreamEndCapture(stream_, &g);
         if (g) cudaGraphDestroy(g);
         cudaGetLastError();
         throw;
       }
-      capturing_ = false;
       GSR_CUDA(cudaStreamEndCapture(stream_, &g));
       cudaGraphExec_t exec = nullptr;
       cudaError_t e = cudaGraphInstantiate(&exec, g, cudaGraphInstantiateFlagUseNodePriority);
@@ -643,7 +616,6 @@ void Pipeline::enqueue(const ViewSpec *views, uint32_t count, uint32_t *images,
   GSR_CUDA(cudaGetLastError());
   last_layout_ = l;
   last_sinks_ = sinks;
-  last_device_sinks_ = device_sinks;
   has_run_ = true;
   last_reused_ = reuse;
   if (!reuse) {
@@ -744,17 +716,14 @@ void Pipeline::enqueue_groups(const ViewSpec *views, uint32_t *images,
         const auto t_capture = std::chrono::steady_clock::now();
         cudaGraph_t g = nullptr;
         GSR_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-        capturing_ = true;
         try {
           launch_groups();
         } catch (...) {
-          capturing_ = false;
           cudaStreamEndCapture(stream_, &g);
           if (g) cudaGraphDestroy(g);
           cudaGetLastError();
           throw;
         }
-        capturing_ = false;
         GSR_CUDA(cudaStreamEndCapture(stream_, &g));
         cudaGraphExec_t exec = nullptr;
         const cudaError_t e = cudaGraphInstantiate(&exec, g, cudaGraphInstantiateFlagUseNodePriority);
@@ -784,29 +753,24 @@ void Pipeline::enqueue_groups(const ViewSpec *views, uint32_t *images,
   GSR_CUDA(cudaGetLastError());
   last_layout_ = layouts.back();
   last_sinks_ = groups.back().sinks;
-  last_device_sinks_ = false;
   has_run_ = true;
   last_reused_ = false;
   sorted_valid_ = false;  // a batch never hands its order to a later frame
 }
 
-void Pipeline::fetch_counters() {
-  if (!last_device_sinks_) return;
-  // the stream is synchronised: counters_ hold the last run's values
-  GSR_CUDA(cudaMemcpy(counters_host_, counters_, sizeof(FrameCounters), cudaMemcpyDeviceToHost));
-  GSR_CUDA(cudaMemcpy(view_counters_pinned_, view_counters_,
-                      sizeof(ViewCounters) * last_layout_.views, cudaMemcpyDeviceToHost));
-  last_sinks_ = HostSinks{counters_host_, view_counters_pinned_};
-}
-
+// By the kernels' own clock readings (the stream is synchronised).
 void Pipeline::phase_times(float out[kPhaseCount]) const {
-  for (int k = 0; k < kPhaseCount; ++k)
-    GSR_CUDA(cudaEventElapsedTime(&out[k], ev_[k], ev_[k + 1]));
+  unsigned long long at = last_sinks_.counters->phase_ns[0];
+  for (int k = 0; k < kPhaseCount; ++k) {
+    const unsigned long long next = std::max(at, last_sinks_.counters->phase_ns[k + 1]);
+    out[k] = (float)((double)(next - at) * 1e-6);
+    at = next;
+  }
 }
 
 void Pipeline::collect(RunResult &r) {
   float t[kPhaseCount];
-  for (int k = 0; k < kPhaseCount; ++k) GSR_CUDA(cudaEventElapsedTime(&t[k], ev_[k], ev_[k + 1]));
+  phase_times(t);
   for (int k = 0; k < kPhaseCount; ++k) r.phase_ms[k] = t[k];
   r.preprocess_ms = t[kPhasePreprocess];
   r.sort_ms = t[kPhaseDepthSort] + t[kPhaseEmit] + t[kPhaseTileSort] + t[kPhaseRanges];
@@ -818,6 +782,17 @@ void Pipeline::collect(RunResult &r) {
   view_counters_host_.assign(last_sinks_.views, last_sinks_.views + last_layout_.views);
 }
 
+// The error bits of the runs since the last call (the stream is synchronised),
+// cleared on both sides.
+uint32_t Pipeline::take_sticky() {
+  const uint32_t sticky = last_sinks_.counters->sticky;
+  if (sticky) {
+    last_sinks_.counters->sticky = 0;
+    GSR_CUDA(cudaMemsetAsync(sticky_, 0, 4, stream_));
+  }
+  return sticky;
+}
+
 RunResult Pipeline::run(const ViewSpec *views, uint32_t count, uint32_t *images,
                         const uint64_t *image_bases) {
   auto t0 = std::chrono::steady_clock::now();
@@ -825,7 +800,6 @@ RunResult Pipeline::run(const ViewSpec *views, uint32_t count, uint32_t *images,
   for (;;) {
     enqueue(views, count, images, image_bases);
     GSR_CUDA(cudaStreamSynchronize(stream_));
-    fetch_counters();
     if (counters_host_->error)
       throw Error(Code::Internal, "device wait limit reached in a look-back scan (error bits " +
                                       std::to_string(counters_host_->error) + ")");
@@ -839,7 +813,7 @@ RunResult Pipeline::run(const ViewSpec *views, uint32_t count, uint32_t *images,
     if (debug_) debug_pairs_.reset(8 * key_cap_, stream_);
     ++r.reruns;
   }
-  GSR_CUDA(cudaMemsetAsync(sticky_, 0, 4, stream_));
+  take_sticky();
   collect(r);
   r.frame_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
   last_ = r;
@@ -848,13 +822,10 @@ RunResult Pipeline::run(const ViewSpec *views, uint32_t count, uint32_t *images,
 
 RunResult Pipeline::sync() {
   GSR_CUDA(cudaSetDevice(device_));
-  uint32_t sticky = 0;
-  GSR_CUDA(cudaMemcpyAsync(&sticky, sticky_, 4, cudaMemcpyDeviceToHost, stream_));
-  GSR_CUDA(cudaMemsetAsync(sticky_, 0, 4, stream_));
   GSR_CUDA(cudaStreamSynchronize(stream_));
   RunResult r;
   if (!has_run_) return r;
-  fetch_counters();
+  const uint32_t sticky = take_sticky();
   collect(r);
   r.frame_ms = r.preprocess_ms + r.sort_ms + r.raster_ms;
   last_ = r;

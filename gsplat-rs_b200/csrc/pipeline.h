@@ -82,7 +82,7 @@ uint64_t scene_device_bytes(const HostScene &s);
 std::unique_ptr<DeviceScene> load_scene_file(const std::string &path, cudaStream_t stream,
                                              const std::function<void(uint64_t)> &admit);
 
-// Device-timed phases of one run (CUDA events on the pipeline's stream).
+// Device-timed phases of one run (the kernels' own clock readings).
 enum Phase : int { kPhasePreprocess, kPhaseDepthSort, kPhaseEmit, kPhaseTileSort, kPhaseRanges,
                    kPhaseRaster, kPhaseCount };
 
@@ -199,11 +199,9 @@ class Pipeline {
   void ensure_key_workspace(uint64_t capacity);
   void launch_all(const Layout &l, uint32_t *images, const HostSinks &sinks, bool reuse,
                   const ViewDev *views_dev, const ViewSetDev *sets_dev);
-  void fetch_counters();  // device-resident counters of the last run -> host (stream synchronised)
+  uint32_t take_sticky();  // stream synchronised
 
  public:
-  // Recorded, in the last enqueued run, just before its raster launch.
-  cudaEvent_t raster_start_event() const { return ev_[kPhaseRaster]; }
   // Phase times of the last run enqueued without batch mode (its stream
   // must have reached the run's end).
   void phase_times(float out[kPhaseCount]) const;
@@ -236,17 +234,15 @@ class Pipeline {
   std::atomic<double> regrowth_ms_{0.0};
   std::atomic<uint64_t> captures_{0};
   std::atomic<double> capture_ms_{0.0};
-  void record(int k);  // phase event k (a graph node while capturing)
 
   int device_;
   cudaStream_t stream_;
   cudaStream_t side_stream_ = nullptr;  // the depth sort; joined into stream_ within every run
   int side_priority_ = 0;               // its priority, the highest
   cudaEvent_t fork_ev_ = nullptr, join_ev_ = nullptr;
-  cudaEvent_t ev_[kPhaseCount + 1] = {};
   uint32_t tile_ = 16, blend_mode_ = 0, sm_count_ = 148;
   RasterConfig raster_cfg_;
-  bool debug_ = false, use_graph_ = true, has_run_ = false, capturing_ = false;
+  bool debug_ = false, use_graph_ = true, has_run_ = false;
   bool reuse_request_ = false, last_reused_ = false, sorted_valid_ = false;
   Layout sorted_layout_;
   std::vector<const DeviceScene *> sorted_scenes_;  // scenes of the last sorted run
@@ -297,7 +293,6 @@ class Pipeline {
   uint64_t table_slot_bytes_ = 0;
   uint64_t table_sets_bytes_ = 0;
   cudaEvent_t slot_ev_[kViewSlots] = {};
-  bool last_device_sinks_ = false;
   int slot_ = 0;
   // CUDA graphs of launch_all, one per layout, buffer set and setting.
   struct GraphKey {
@@ -356,7 +351,7 @@ class Pipeline {
   unsigned char *batch_stage_ = nullptr;  // pinned: every group's view table, back to back
   uint64_t batch_stage_bytes_ = 0;
   cudaEvent_t batch_ev_ = nullptr;        // the last batch launch has read the staging area
-  bool batch_mode_ = false;               // launch_all: table copied, no phase events
+  bool batch_mode_ = false;               // launch_all: table copied, no end of the raster noted
   uint64_t batch_graph_launches_ = 0;
   void drop_batch_graphs();
   uint64_t graph_clock_ = 0;

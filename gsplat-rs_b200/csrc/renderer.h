@@ -151,7 +151,7 @@ class Renderer {
     uint8_t *out = nullptr;
     uint64_t bytes = 0;
   } deferred_;
-  void issue_copy(bool after_next_raster);
+  void issue_copy();
   const std::vector<uint64_t> image_base_{0};
 };
 

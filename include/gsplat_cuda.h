@@ -320,7 +320,7 @@ int32_t gsplat_batch_render(GsplatBatch *batch, const GsplatBatchView *views, ui
 int32_t gsplat_batch_get_times(const GsplatBatch *batch, GsplatBatchTimes *out_times);
 /* Phase timing (off by default): while on, a render runs its launch groups one
  * after another, waiting after each, in place of the whole-batch graph, and
- * records per-phase CUDA-event times summed over the groups. A measurement
+ * records per-phase device times summed over the groups. A measurement
  * mode: the images are the same, the device time is not the production one. */
 int32_t gsplat_batch_set_phase_timing(GsplatBatch *batch, uint32_t on);
 /* Per-phase device ms of the last render, in the order preprocess, depth sort,
