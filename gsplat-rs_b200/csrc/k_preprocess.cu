@@ -20,6 +20,7 @@
 
 #include "device_common.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace gsr {
 
@@ -727,9 +728,10 @@ void launch_k1(const ViewDev *views, const ViewSetDev *sets, uint32_t num_sets,
 uint32_t key_blocks(uint32_t splats) { return (splats + kKeyTile - 1) / kKeyTile; }
 
 void launch_keys(const ViewDev *views, const ViewSetDev *sets, uint32_t num_sets,
-                 uint32_t total_blocks, const K1Buffers &b, cudaStream_t stream) {
+                 uint32_t total_blocks, const K1Buffers &b, int priority, cudaStream_t stream) {
   if (total_blocks == 0) return;
-  keys_kernel<<<total_blocks, kK1Threads, 0, stream>>>(views, sets, num_sets, total_blocks, b);
+  launch_kernel(keys_kernel, total_blocks, kK1Threads, 0, priority, stream, views, sets, num_sets,
+                total_blocks, b);
 }
 
 uint32_t preprocess_blocks(uint32_t splats) { return (splats + kK1Threads - 1) / kK1Threads; }

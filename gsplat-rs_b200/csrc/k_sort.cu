@@ -24,6 +24,7 @@
 
 #include "device_common.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace gsr {
 namespace {
@@ -634,21 +635,10 @@ uint32_t device_sm_count() {
 }
 
 namespace {
-// Launches a kernel of the sort at the sort's priority. The priority of a
-// captured launch is the launch's own, not its stream's.
 template <typename... P, typename... A>
 void launch_at(const SortBuffers &b, void (*kernel)(P...), uint32_t grid, cudaStream_t stream,
                A... args) {
-  cudaLaunchConfig_t c{};
-  c.gridDim = dim3(grid);
-  c.blockDim = dim3(kThreads);
-  c.stream = stream;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributePriority;
-  attr.val.priority = b.priority;
-  c.attrs = &attr;
-  c.numAttrs = 1;
-  cudaLaunchKernelEx(&c, kernel, P(args)...);
+  launch_kernel(kernel, grid, kThreads, 0, b.priority, stream, args...);
 }
 
 // The one pass of a wide sort; the histograms are given.

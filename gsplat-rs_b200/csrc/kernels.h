@@ -40,7 +40,7 @@ uint32_t preprocess_blocks(uint32_t splats);
 uint32_t key_blocks(uint32_t splats);
 // The depth keys and ids of the visible splats, their count and histograms.
 void launch_keys(const ViewDev *views, const ViewSetDev *sets, uint32_t num_sets,
-                 uint32_t total_blocks, const K1Buffers &b, cudaStream_t stream);
+                 uint32_t total_blocks, const K1Buffers &b, int priority, cudaStream_t stream);
 // The records and rects; independent of the keys.
 void launch_preprocess(const ViewDev *views, const ViewSetDev *sets, uint32_t num_sets,
                        uint32_t total_blocks, uint32_t max_planes, const K1Buffers &b, bool debug,
