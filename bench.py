@@ -187,19 +187,36 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(sel), "selection": how}
 
 
-def algorithmic_bytes(phase, counts, n, planes, width, height, tile_passes):
-    """Bytes each phase must move at minimum (reads + writes), per frame."""
+def view_bins(width, height, tile=16):
+    """Bins (4x4 tiles) of a view's image."""
+    edge = 4 * tile
+    return ((width + edge - 1) // edge) * ((height + edge - 1) // edge)
+
+
+def bin_passes(bins):
+    """Passes of the bin sort: one up to 1,024 bins, else 8 bits a pass."""
+    passes = 1
+    while bins > 1024 and (1 << (8 * passes)) < bins:
+        passes += 1
+    return passes
+
+
+def algorithmic_bytes(phase, counts, n, planes, width, height, passes):
+    """Bytes each phase must move at minimum (reads + writes), per frame. The
+    sorted pairs are (4x4-tile bin, splat) pairs, at least a sixteenth of the
+    tile pairs."""
     v, d, k = counts.visible, counts.drawn, counts.tile_keys
+    b = k // 16
     if phase == "preprocess":
         return n * 16 + v * 32 + d * 16 * planes + v * 16 + d * 48
     if phase == "depth_sort":
-        return v * 4 + 3 * v * 16  # histogram read + three non-trivial passes
+        return 3 * v * 16  # three non-trivial passes
     if phase == "emit":
-        return v * 4 + v * 8 + k * 8
+        return v * 4 + v * 8 + d * 32 + b * 8
     if phase == "tile_sort":
-        return k * 4 + tile_passes * k * 16
+        return passes * b * 16
     if phase == "ranges":
-        return k * 4
+        return b * 6
     if phase == "raster":
         return k * 52 + width * height * 4
     return 0
@@ -446,17 +463,11 @@ def measure_batched(ffi, torch, steps, warmup, cameras_per_scene=64):
     phase_ms = b.phase_times()
     b.set_phase_timing(False)
     stats = [b.view_stats(k) for k in range(len(specs))]
-    group_tiles = {}
+    group_bins = {}
     for k, (sid, _, w, h) in enumerate(specs):
         g = stats[k].group
-        group_tiles[g] = group_tiles.get(g, 0) + ((w + 15) // 16) * ((h + 15) // 16)
-    group_passes = {}
-    for g, tiles in group_tiles.items():
-        p = 1
-        while (1 << (8 * p)) < tiles:
-            p += 1
-        group_passes[g] = p
-    hbm = hbm_peak_gbs()
+        group_bins[g] = group_bins.get(g, 0) + view_bins(w, h)
+    group_passes = {g: bin_passes(bins) for g, bins in group_bins.items()}
     phases = {}
     for k, ms in phase_ms.items():
         if k == "preprocess":
@@ -531,10 +542,10 @@ def measure_batched(ffi, torch, steps, warmup, cameras_per_scene=64):
             "per_scene": per_scene,
             "phases": phases, "phases_hbm_peak_gbs": hbm[0], "phases_hbm_peak_source": hbm[1],
             "phases_timing": "a separate phase-timed render of the same batch "
-                             "(gsplat_batch_set_phase_timing): per-phase CUDA events of each "
+                             "(gsplat_batch_set_phase_timing): per-phase device times of each "
                              "launch group, summed; groups run one by one",
             "timing": "device ms from CUDA events around all launch groups (batched) and the "
-                      "per-phase CUDA events of each plain frame; scenes exceed L2"}
+                      "per-phase device times of each plain frame; scenes exceed L2"}
 
 
 def _spin_until(t):
@@ -873,10 +884,7 @@ def measure_config3(ffi, torch, frames=20):
     hbm = peaks.get("hbm_gbs") or FALLBACK_HBM_GBS
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.int32, device="cuda")
     n = scene["positions"].shape[0]
-    tiles = ((w + 15) // 16) * ((h + 15) // 16)
-    tile_passes = 1
-    while (1 << (8 * tile_passes)) < tiles:
-        tile_passes += 1
+    passes = bin_passes(view_bins(w, h))
     out = {"workload": "3,000,000 synthetic splats, SH degree 3, uniform 10^3 box + dense core, "
                        "camera inside the volume, 3840x2160, 16x16 tiles",
            "hbm_peak_gbs": hbm, "hbm_peak_source": "measured" if peaks.get("hbm_gbs") else "fallback",
@@ -900,7 +908,7 @@ def measure_config3(ffi, torch, frames=20):
             ph = {k: float(np.median(v)) for k, v in acc.items()}
             phases = {}
             for k, ms in ph.items():
-                b = algorithmic_bytes(k, counts, n, 12, w, h, tile_passes)
+                b = algorithmic_bytes(k, counts, n, 12, w, h, passes)
                 gbs = b / (ms * 1e-3) / 1e9 if ms > 0 else None
                 phases[k] = {"ms": ms, "bytes": b, "gbs": gbs,
                              "frac_measured": gbs / hbm if gbs else None,
@@ -1063,8 +1071,7 @@ def run_cuda(args, world, rank, local):
            "frame_lanes": args.frame_lanes,
            "single_lane_value": whole_job_rate(world, args.steps, e2e_single_s)}
 
-    tiles = ((w + 15) // 16) * ((h + 15) // 16)
-    tile_passes = 2 if tiles > 256 else 1
+    passes = bin_passes(view_bins(w, h))
     planes = 12
     dominant = max(phases, key=phases.get)
     peaks = {}
@@ -1073,7 +1080,7 @@ def run_cuda(args, world, rank, local):
             peaks = json.load(f)
     hbm = peaks.get("hbm_gbs")
     bytes_dom = algorithmic_bytes(dominant, counts, scene["positions"].shape[0], planes, w, h,
-                                  tile_passes)
+                                  passes)
     achieved = bytes_dom / (phases[dominant] * 1e-3) / 1e9
     peak = hbm if hbm else FALLBACK_HBM_GBS
     roofline = {"kernel": dominant, "bound": "hbm", "achieved": achieved, "peak": peak,
@@ -1101,13 +1108,13 @@ def run_cuda(args, world, rank, local):
             roofline["counters_source"] = NCU_RASTER["source"]
     phase_rooflines = {}
     for k, ms in phases.items():
-        b = algorithmic_bytes(k, counts, scene["positions"].shape[0], planes, w, h, tile_passes)
+        b = algorithmic_bytes(k, counts, scene["positions"].shape[0], planes, w, h, passes)
         phase_rooflines[k] = {"ms": ms, "bytes": b, "gbs": b / (ms * 1e-3) / 1e9 if ms > 0 else None}
 
-    # scratch zeroing; preprocess; depth sort: plan + 4 passes (histograms
-    # from K1); emit; tile sort: plan + passes (histograms from K2); ranges;
-    # raster
-    launches_per_frame = 1 + 1 + (1 + 4) + 1 + (1 + tile_passes) + 1 + 1
+    # scratch zeroing; keys; depth sort: plan + 4 passes (histograms from the
+    # keys); vertex stage; emit; bin sort: plan + passes (histograms from the
+    # emission); ranges; raster
+    launches_per_frame = 1 + 1 + (1 + 4) + 1 + 1 + (1 + passes) + 1 + 1
     line = {"metric": METRIC, "value": value, "unit": "frames/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_per_frame,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",

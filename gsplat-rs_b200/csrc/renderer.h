@@ -86,8 +86,8 @@ class Renderer {
   void readback_rgba8(uint8_t *out, uint64_t len);
   // Requests the copy of the last frame's image into `out` (pinned host
   // memory, kept valid until sync()) and returns. The copy runs on a copy
-  // stream while the next frame renders: it is issued with that frame, timed
-  // to its raster, or at sync(). Frames alternate between two image buffers;
+  // stream while the next frame renders: it is issued behind that frame's
+  // launches, or at sync(). Frames alternate between two image buffers;
   // a buffer is rendered into again only after its copy.
   void readback_rgba8_async(uint8_t *out, uint64_t len);
   std::vector<uint32_t> debug_order();
@@ -142,9 +142,9 @@ class Renderer {
   cudaEvent_t rendered_[kMaxLanes] = {};  // the frame into image_[k] is complete
   cudaEvent_t copied_[kMaxLanes] = {};    // the async readback of image_[k] is complete
   bool copy_pending_[kMaxLanes] = {};
-  // A readback requested but not yet issued: it starts with the next frame's
-  // raster (one long kernel, so the copy's PCIe traffic does not delay that
-  // frame's other launches), or at sync().
+  // A readback requested but not yet issued: it is issued behind the next
+  // frame's launches, so a destination that blocks the call (pageable memory)
+  // does not hold that frame up, or at sync().
   struct DeferredCopy {
     bool pending = false;
     int image = 0;
