@@ -52,7 +52,7 @@ def bench_config(world):
             "parallelism": f"CUDA arm: one replica per GPU (x{world}), no collective on the "
                            "data path; CPU arm: host threads on rank 0"}
 FALLBACK_HBM_GBS = 6650.0
-# Per-launch counters of the 1080p raster (raster_fp32_kernel<16, 256>) from
+# Per-launch counters of the 1080p raster (raster_fp32_kernel<16, 128, 2, 8>) from
 # one ncu capture of this workload (profiles/frame_279k_sh3_1080p.md gives
 # the command): DRAM bytes read + written, warp instructions issued, and
 # executed FP32 thread operations (2 x FFMA + FADD + FMUL). None until
@@ -61,9 +61,9 @@ FALLBACK_HBM_GBS = 6650.0
 # same arithmetic (-D GSR_RASTER_F32X2=0; ncu's per-op counters do not count
 # the paired f32x2 instructions of the default build, which performs exactly
 # the same operations).
-NCU_RASTER = {"dram_bytes": 18_311_168, "warp_inst": 95_671_016,
-              "thread_flop": 2 * 1_223_868_317 + 202_085_090 + 375_960_460,
-              "source": "profiles/frame_279k_sh3_1080p.md (ncu --set full, one launch)"}
+NCU_RASTER = {"dram_bytes": 14_561_024, "warp_inst": 90_028_672,
+              "thread_flop": 2 * 1_265_338_181 + 172_377_046 + 329_943_846,
+              "source": "profiles/frame_279k_sh3_1080p.md (ncu, one launch)"}
 
 
 def dist_setup():
