@@ -468,6 +468,7 @@ def measure_batched(ffi, torch, steps, warmup, cameras_per_scene=64):
         g = stats[k].group
         group_bins[g] = group_bins.get(g, 0) + view_bins(w, h)
     group_passes = {g: bin_passes(bins) for g, bins in group_bins.items()}
+    hbm = hbm_peak_gbs()
     phases = {}
     for k, ms in phase_ms.items():
         if k == "preprocess":
