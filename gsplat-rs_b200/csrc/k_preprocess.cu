@@ -699,15 +699,7 @@ void launch_k1_t(const ViewDev *views, const ViewSetDev *sets, uint32_t num_sets
                  uint32_t total_blocks, const K1Buffers &b, cudaStream_t stream) {
   constexpr size_t kSmem = sizeof(K1Stage<kPlanes>);
   constexpr size_t kMost = kSmem > kTwoBlockSmem ? kSmem : kTwoBlockSmem;
-  static const bool configured = [] {
-    cudaFuncSetAttribute(preprocess_kernel<kPlanes, kDebug>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost);
-    cudaFuncSetAttribute(preprocess_kernel<kPlanes, kDebug>,
-                         cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
-    return true;
-  }();
-  (void)configured;
+  allow_shared_memory<preprocess_kernel<kPlanes, kDebug>>((int)kMost, true);
   const size_t smem = total_blocks <= kTwoBlockTiles && !b.reuse_order ? kMost : kSmem;
   preprocess_kernel<kPlanes, kDebug>
       <<<total_blocks, kK1Threads, smem, stream>>>(views, sets, num_sets, b);

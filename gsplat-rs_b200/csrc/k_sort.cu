@@ -592,15 +592,6 @@ uint64_t sort_work_words(uint32_t capacity, uint32_t passes) {
 }
 
 namespace {
-constexpr int kMaxDevices = 64;
-int current_device() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
-    cudaGetLastError();
-    dev = 0;
-  }
-  return dev;
-}
 // Resident pass blocks on the current device (the persistent grid), looked
 // up once per device.
 template <auto kKernel>

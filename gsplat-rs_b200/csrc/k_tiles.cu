@@ -24,6 +24,7 @@
 #include "bins.cuh"
 #include "device_common.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 #include "tile_span.cuh"
 
 namespace gsr {
@@ -458,17 +459,14 @@ void launch_emit(const EmitBuffers &b, cudaStream_t stream) {
   if (blocks == 0 || b.num_views == 0) return;
   const size_t smem = 4 * 4 * b.num_views;
   // The static arrays and the largest view table together pass 48 KB.
-  static const bool configured = [] {
-    const int most = (int)(4 * 4 * kMaxViewsPerLaunch);
-    cudaFuncSetAttribute(emit_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    cudaFuncSetAttribute(emit_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    return true;
-  }();
-  (void)configured;
-  if (emit_ipt(b.n) == 2)
+  constexpr int kMost = (int)(4 * 4 * kMaxViewsPerLaunch);
+  if (emit_ipt(b.n) == 2) {
+    allow_shared_memory<emit_kernel<2>>(kMost);
     emit_kernel<2><<<blocks, kEmitThreads, smem, stream>>>(b);
-  else
+  } else {
+    allow_shared_memory<emit_kernel<4>>(kMost);
     emit_kernel<4><<<blocks, kEmitThreads, smem, stream>>>(b);
+  }
 }
 
 void launch_ranges(const SortPlan *bin_plan, uint32_t *keys0, uint32_t *keys1,

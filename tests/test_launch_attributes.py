@@ -1,0 +1,39 @@
+"""What the kernel launches ask of the CUDA runtime, on a stand-in with two
+devices (tests/ffi/launch_probe.cpp): no GPU is needed."""
+
+import os
+import subprocess
+
+import pytest
+
+import build as native
+from conftest import ROOT
+
+OBJECTS = ("k_preprocess.cu.o", "k_tiles.cu.o", "k_sort.cu.o")
+
+
+@pytest.fixture(scope="module")
+def probe(tmp_path_factory):
+    native.build()
+    exe = str(tmp_path_factory.mktemp("probe") / "launch_probe")
+    subprocess.run([native.CXX, "-std=c++17", "-O1", "-I", native.CSRC, "-I", native.INCLUDE,
+                    "-I", os.path.join(native.CUDA_HOME, "include"),
+                    os.path.join(ROOT, "tests", "ffi", "launch_probe.cpp"),
+                    *[os.path.join(native.BUILD, o) for o in OBJECTS], "-o", exe], check=True)
+
+    def run(what):
+        out = subprocess.run([exe, what], capture_output=True, text=True, check=True).stdout
+        rows = [line.split()[1:] for line in out.splitlines() if line.startswith("launch ")]
+        return [(int(d), int(smem), int(limit), prio) for d, smem, limit, prio in rows]
+
+    return run
+
+
+@pytest.mark.parametrize("what", ["preprocess", "emit"])
+def test_shared_memory_limits_are_raised_on_every_device(probe, what):
+    """A kernel's dynamic shared memory limit belongs to a device: each device
+    a process renders on has to get it, not the first one alone."""
+    launches = probe(what)
+    by_device = [[l[1:] for l in launches if l[0] == d] for d in (0, 1)]
+    assert by_device[0] and by_device[0] == by_device[1]
+    assert all(smem <= limit for _, smem, limit, _ in launches), launches
