@@ -720,7 +720,8 @@ void launch_k1(const ViewDev *views, const ViewSetDev *sets, uint32_t num_sets,
 uint32_t key_blocks(uint32_t splats) { return (splats + kKeyTile - 1) / kKeyTile; }
 
 void launch_keys(const ViewDev *views, const ViewSetDev *sets, uint32_t num_sets,
-                 uint32_t total_blocks, const K1Buffers &b, int priority, cudaStream_t stream) {
+                 uint32_t total_blocks, const K1Buffers &b, std::optional<int> priority,
+                 cudaStream_t stream) {
   if (total_blocks == 0) return;
   launch_kernel(keys_kernel, total_blocks, kK1Threads, 0, priority, stream, views, sets, num_sets,
                 total_blocks, b);

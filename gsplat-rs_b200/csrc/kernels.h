@@ -3,6 +3,7 @@
 
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <optional>
 
 #include "device_types.h"
 #include "gsr_host.h"
@@ -40,7 +41,8 @@ uint32_t preprocess_blocks(uint32_t splats);
 uint32_t key_blocks(uint32_t splats);
 // The depth keys and ids of the visible splats, their count and histograms.
 void launch_keys(const ViewDev *views, const ViewSetDev *sets, uint32_t num_sets,
-                 uint32_t total_blocks, const K1Buffers &b, int priority, cudaStream_t stream);
+                 uint32_t total_blocks, const K1Buffers &b, std::optional<int> priority,
+                 cudaStream_t stream);
 // The records and rects; independent of the keys.
 void launch_preprocess(const ViewDev *views, const ViewSetDev *sets, uint32_t num_sets,
                        uint32_t total_blocks, uint32_t max_planes, const K1Buffers &b, bool debug,
@@ -71,7 +73,7 @@ struct SortBuffers {
   // 9 or 10: one pass over that many bits (passes = 1, histograms given, and
   // sort_work_words of 4 passes).
   uint32_t wide_bits = 0;
-  int priority = 0;  // launch priority of the kernels (as a stream's)
+  std::optional<int> priority;  // launch priority of the kernels (default: the stream's)
   unsigned long long *start_ns = nullptr;  // when the sort starts, if wanted
 };
 constexpr uint32_t kSortScratchHeadWords = 64 + 4 * 256;  // tickets and histograms

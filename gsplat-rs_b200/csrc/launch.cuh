@@ -6,6 +6,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <optional>
 
 namespace gsr {
 
@@ -36,21 +37,24 @@ void allow_shared_memory(int bytes, bool max_carveout = false) {
   if (e == cudaSuccess) done[dev].store(true, std::memory_order_relaxed);
 }
 
-// A kernel launch with a priority of its own. The priority of a captured launch
-// is the launch's, not its stream's.
+// A kernel launch, with a priority of its own where one is given (the priority
+// of a captured launch is the launch's, not its stream's). Without one it runs
+// at its stream's: a sort on a caller's stream keeps that stream's priority.
 template <typename... P, typename... A>
 void launch_kernel(void (*kernel)(P...), uint32_t grid, uint32_t threads, size_t smem,
-                   int priority, cudaStream_t stream, A... args) {
+                   std::optional<int> priority, cudaStream_t stream, A... args) {
   cudaLaunchConfig_t c{};
   c.gridDim = dim3(grid);
   c.blockDim = dim3(threads);
   c.dynamicSmemBytes = smem;
   c.stream = stream;
   cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributePriority;
-  attr.val.priority = priority;
-  c.attrs = &attr;
-  c.numAttrs = 1;
+  if (priority) {
+    attr.id = cudaLaunchAttributePriority;
+    attr.val.priority = *priority;
+    c.attrs = &attr;
+    c.numAttrs = 1;
+  }
   cudaLaunchKernelEx(&c, kernel, P(args)...);
 }
 

@@ -444,7 +444,7 @@ void Pipeline::launch_all(const Layout &l, uint32_t *images, const HostSinks &si
   // blocks that wait for one another, the vertex stage many that do not). The
   // keys beside it too: 3M splats 1,495 -> 1,480 us, 64 thumbnails 457 -> 451.
   if (reuse) {  // a reused order keeps the last sort's ids and plan
-    launch_keys(views_dev, sets_dev, l.sets, l.key_blocks, k1, 0, stream_);
+    launch_keys(views_dev, sets_dev, l.sets, l.key_blocks, k1, std::nullopt, stream_);
   } else {
     GSR_CUDA(cudaEventRecord(fork_ev_, stream_));
     GSR_CUDA(cudaStreamWaitEvent(side_stream_, fork_ev_, 0));

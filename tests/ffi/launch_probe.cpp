@@ -2,7 +2,7 @@
 // devices: no GPU, no kernel runs. Prints one line per launch: the device, the
 // dynamic shared memory it asks for, the limit raised for that kernel on that
 // device (0: none), and the launch's priority attribute ("-": none).
-//   launch_probe preprocess|emit|sort
+//   launch_probe preprocess|emit|sort|sort-high
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -101,11 +101,17 @@ int main(int argc, char **argv) {
         b.num_views = kMaxViewsPerLaunch;
         launch_emit(b, nullptr);
       }
-    } else if (!std::strcmp(what, "sort")) {
+    } else if (!std::strncmp(what, "sort", 4)) {
+      const bool high = !std::strcmp(what, "sort-high");
+      const uint32_t hist[1] = {};
       for (uint32_t bits : {0u, 9u, 10u})
         for (uint32_t capacity : {1000u, 1u << 22, 1u << 25}) {
           SortBuffers b{};
           b.capacity = capacity;
+          if (high) {  // as a frame's depth sort: histograms given, a priority asked for
+            b.hist = hist;
+            b.priority = -5;
+          }
           b.passes = bits ? 1 : 4;
           b.wide_bits = bits;
           launch_sort(b, nullptr);

@@ -37,3 +37,12 @@ def test_shared_memory_limits_are_raised_on_every_device(probe, what):
     by_device = [[l[1:] for l in launches if l[0] == d] for d in (0, 1)]
     assert by_device[0] and by_device[0] == by_device[1]
     assert all(smem <= limit for _, smem, limit, _ in launches), launches
+
+
+def test_sorts_keep_the_priority_of_their_stream(probe):
+    """A sort asks for no priority unless its caller did: on a stream with a
+    priority of its own every kernel of it then runs at that priority."""
+    launches = probe("sort")
+    assert len(launches) >= 2 * 9 and all(prio == "-" for *_, prio in launches), launches
+    asked = probe("sort-high")
+    assert asked and all(prio == "-5" for *_, prio in asked), asked
