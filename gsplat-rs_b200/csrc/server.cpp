@@ -7,6 +7,8 @@
 #include <cmath>
 #include <cstring>
 
+#include <sys/prctl.h>
+
 #include "cuda_check.h"
 #include "kernels.h"
 #include "renderer.h"
@@ -528,9 +530,11 @@ void Server::retire(LaneState &ls, std::unique_lock<std::mutex> &lk) {
 
 void Server::loop() {
   cudaSetDevice(device_);
+  prctl(PR_SET_TIMERSLACK, 1000);  // this thread's short sleeps end on time (1 us, not 50)
   std::unique_lock<std::mutex> lk(mu_);
   while (true) {
     bool progressed = false;
+    double hold = 0;
     for (auto &ls : lanes_)
       if (ls->busy && ls->completed.load()) {
         retire(*ls, lk);
@@ -542,9 +546,23 @@ void Server::loop() {
       if (!any_busy) break;
     } else {
       for (auto &ls : lanes_)
-        if (!ls->busy && !queue_.empty()) progressed |= launch(*ls, lk);
+        if (!ls->busy && !queue_.empty()) {
+          bool device_busy = false;
+          for (auto &o : lanes_) device_busy |= o->busy;
+          hold = gather_ms(now_ms(), requests_.at(queue_.front()).t_submit,
+                           requests_.at(queue_.back()).t_submit, device_busy,
+                           queue_.size() >= cfg_.max_views);
+          if (hold > 0) break;
+          progressed |= launch(*ls, lk);
+        }
     }
-    if (!progressed) cv_.wait(lk);
+    if (hold > 0) {
+      lk.unlock();  // submits go on
+      std::this_thread::sleep_for(std::chrono::duration<double, std::milli>(hold));
+      lk.lock();
+    } else if (!progressed) {
+      cv_.wait(lk);
+    }
   }
   // fail whatever is still queued
   for (uint64_t id : queue_) {
