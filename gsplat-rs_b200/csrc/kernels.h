@@ -78,6 +78,11 @@ struct SortBuffers {
 };
 constexpr uint32_t kSortScratchHeadWords = 64 + 4 * 256;  // tickets and histograms
 uint64_t sort_work_words(uint32_t capacity, uint32_t passes);
+// The pair buffers' sort has scratch for any bin count: four passes, or as many
+// words as a wide pass takes, 2 bytes per pair. A pair's workspace is that and
+// its key and value in two buffers.
+constexpr uint32_t kPairSortPasses = 4;
+constexpr uint64_t kPairWorkspaceBytes = 18;
 // Zeroes the scratch (one memset) and launches the histogram (unless given),
 // plan and pass kernels on `stream`.
 void launch_sort(const SortBuffers &b, cudaStream_t stream);

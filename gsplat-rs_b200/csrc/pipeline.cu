@@ -376,7 +376,6 @@ void Pipeline::ensure_workspace(const Layout &l) {
 }
 
 void Pipeline::ensure_key_workspace(uint64_t capacity) {
-  const uint32_t passes = 4;  // enough for any bin count (a wide pass takes as many words)
   if (key_cap_ >= capacity && key_ws_.get()) return;
   if (capacity > kMaxSortItems)
     throw Error(Code::Unsupported, "tile pair count " + std::to_string(capacity) +
@@ -387,7 +386,7 @@ void Pipeline::ensure_key_workspace(uint64_t capacity) {
   // geometric growth, as for the other workspaces
   const uint32_t cap = (uint32_t)std::min<uint64_t>(
       std::max<uint64_t>(capacity, key_cap_ + key_cap_ / 4), kMaxSortItems);
-  const uint64_t words = sort_work_words(cap, passes);
+  const uint64_t words = sort_work_words(cap, kPairSortPasses);
   uint64_t off = 0;
   uint64_t o_k0 = off; off += align256(4ull * cap);
   uint64_t o_v0 = off; off += align256(4ull * cap);

@@ -341,9 +341,9 @@ void Server::reset_stats() {
 }
 
 uint64_t Server::view_bytes(const ViewSpec &s, uint64_t pairs) const {
-  // pair keys and values, double-buffered, plus sort scratch; splat
-  // workspace (keys, ids, rect, record, sort scratch); the image
-  return pairs * 17 + (uint64_t)s.scene->n * 80 + 4ull * s.width * s.height;
+  // the pairs' workspace; splat workspace (keys, ids, rect, record, sort
+  // scratch); the image
+  return pairs * kPairWorkspaceBytes + (uint64_t)s.scene->n * 80 + 4ull * s.width * s.height;
 }
 
 void Server::on_lane_done(void *arg) {

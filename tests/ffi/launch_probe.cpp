@@ -3,6 +3,8 @@
 // dynamic shared memory it asks for, the limit raised for that kernel on that
 // device (0: none), and the launch's priority attribute ("-": none).
 //   launch_probe preprocess|emit|sort|sort-high
+// "work" prints pair capacities, the words of their sort's scratch and the bytes
+// a pair is counted with in place of launches.
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -116,6 +118,11 @@ int main(int argc, char **argv) {
           b.wide_bits = bits;
           launch_sort(b, nullptr);
         }
+    } else if (!std::strcmp(what, "work")) {
+      for (uint32_t capacity : {1u << 20, 3'000'001u, 1u << 28})
+        std::printf("work %u %llu %llu\n", capacity,
+                    (unsigned long long)sort_work_words(capacity, kPairSortPasses),
+                    (unsigned long long)kPairWorkspaceBytes);
     } else {
       return 2;
     }

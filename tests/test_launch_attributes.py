@@ -21,11 +21,15 @@ def probe(tmp_path_factory):
                     os.path.join(ROOT, "tests", "ffi", "launch_probe.cpp"),
                     *[os.path.join(native.BUILD, o) for o in OBJECTS], "-o", exe], check=True)
 
-    def run(what):
+    def lines(what, kind):
         out = subprocess.run([exe, what], capture_output=True, text=True, check=True).stdout
-        rows = [line.split()[1:] for line in out.splitlines() if line.startswith("launch ")]
-        return [(int(d), int(smem), int(limit), prio) for d, smem, limit, prio in rows]
+        return [line.split()[1:] for line in out.splitlines() if line.startswith(kind + " ")]
 
+    def run(what):
+        return [(int(d), int(smem), int(limit), prio)
+                for d, smem, limit, prio in lines(what, "launch")]
+
+    run.values = lambda what: [tuple(map(int, row)) for row in lines(what, "work")]
     return run
 
 
@@ -46,3 +50,10 @@ def test_sorts_keep_the_priority_of_their_stream(probe):
     assert len(launches) >= 2 * 9 and all(prio == "-" for *_, prio in launches), launches
     asked = probe("sort-high")
     assert asked and all(prio == "-5" for *_, prio in asked), asked
+
+
+def test_admitted_pair_bytes_cover_the_workspace(probe):
+    """What the server counts per pair is at least what a lane allocates: keys
+    and values twice and the sort's scratch."""
+    for capacity, words, counted in probe.values("work"):
+        assert 16 * capacity + 4 * words <= counted * capacity + (1 << 16), (capacity, words)
