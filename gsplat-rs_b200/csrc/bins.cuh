@@ -80,5 +80,17 @@ constexpr uint32_t kWordGroup = 8;
 GSR_HD uint64_t tile_word(uint32_t w, uint32_t t) {
   return ((uint64_t)(w / kWordGroup) * kBinTiles + t) * kWordGroup + w % kWordGroup;
 }
+// Words of the tiles of n list positions.
+GSR_HD uint64_t tile_words(uint64_t n) {
+  return (n + 32 * kWordGroup - 1) / (32 * kWordGroup) * (kBinTiles * kWordGroup);
+}
+
+// each(position) for the list positions [first, end) that have tile `t`, by the
+// range build's words: a tile's list as the raster takes it.
+template <typename F>
+void each_tile_position(const uint32_t *words, uint32_t first, uint32_t end, uint32_t t, F each) {
+  for (uint64_t i = first; i < end; ++i)
+    if (words[tile_word((uint32_t)(i / 32), t)] >> (i % 32) & 1u) each((uint32_t)i);
+}
 
 }  // namespace gsr

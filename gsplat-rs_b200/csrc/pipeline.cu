@@ -923,45 +923,39 @@ void Pipeline::debug_tile_pairs(std::vector<uint32_t> &tiles, std::vector<uint32
   }
 }
 
-// Every tile's list, as the raster takes it from its bin's.
+// Every tile's list, from what the raster reads: the bins' ranges, the tiles'
+// words (in the key buffer the sort has left free) and the sorted ids.
 void Pipeline::debug_tile_ranges(uint32_t num_tiles, std::vector<uint32_t> &ranges,
                                  std::vector<uint32_t> &ids) {
   GSR_CUDA(cudaSetDevice(device_));
   SortPlan plan = read_plan(1);
+  const bool first = plan.final_buffer == 0;
   const uint64_t n = std::min<uint64_t>(last_sinks_.counters->pairs, key_cap_);
-  std::vector<uint32_t> keys(n), vals(n);
-  if (n) {
-    const bool first = plan.final_buffer == 0;
-    GSR_CUDA(cudaMemcpy(keys.data(), first ? pair_keys0_ : pair_keys1_, 4 * n,
-                        cudaMemcpyDeviceToHost));
-    GSR_CUDA(cudaMemcpy(vals.data(), first ? pair_vals0_ : pair_vals1_, 4 * n,
-                        cudaMemcpyDeviceToHost));
-  }
-  const uint32_t tiles_x = views_host_[0].p.tiles_x, bins_x = bins_along(tiles_x);
-  std::vector<uint32_t> count(num_tiles, 0);
-  auto each = [&](auto f) {
-    for (uint64_t k = 0; k < n; ++k) {
-      const uint32_t bin = keys[k] >> kBinCodeBits;
-      for (uint32_t r = 0; r < kBinEdge; ++r)
-        for (uint32_t c = 0; c < kBinEdge; ++c)
-          if (bin_code_tiles(keys[k]) >> (kBinEdge * r + c) & 1u)
-            f((bin / bins_x * kBinEdge + r) * tiles_x + bin % bins_x * kBinEdge + c, vals[k]);
-    }
+  const FrameParams &p = views_host_[0].p;
+  const uint32_t bins_x = bins_along(p.tiles_x);
+  std::vector<uint32_t> words(tile_words(n)), sorted(n);
+  std::vector<uint2> bin_ranges((size_t)bins_x * bins_along(p.tiles_y));
+  auto fetch = [](auto &to, const void *from) {
+    if (!to.empty())
+      GSR_CUDA(cudaMemcpy(to.data(), from, sizeof(to[0]) * to.size(), cudaMemcpyDeviceToHost));
   };
-  each([&](uint32_t t, uint32_t) { ++count[t]; });
+  fetch(words, first ? pair_keys1_ : pair_keys0_);
+  fetch(sorted, first ? pair_vals0_ : pair_vals1_);
+  fetch(bin_ranges, ranges_);
   ranges.assign(2ull * num_tiles, 0);
-  uint32_t at = 0;
-  for (uint32_t t = 0; t < num_tiles; ++t) {
-    if (count[t]) {
+  ids.clear();
+  for (uint32_t t = 0; t < std::min(num_tiles, p.num_tiles); ++t) {
+    const uint32_t tx = t % p.tiles_x, ty = t / p.tiles_x;
+    const uint2 r = bin_ranges[ty / kBinEdge * bins_x + tx / kBinEdge];
+    const uint32_t at = (uint32_t)ids.size();
+    each_tile_position(words.data(), r.x, std::min<uint32_t>(r.y, (uint32_t)n),
+                       ty % kBinEdge * kBinEdge + tx % kBinEdge,
+                       [&](uint32_t i) { ids.push_back(sorted[i]); });
+    if (ids.size() > at) {
       ranges[2ull * t] = at;
-      ranges[2ull * t + 1] = at + count[t];
+      ranges[2ull * t + 1] = (uint32_t)ids.size();
     }
-    const uint32_t c = count[t];
-    count[t] = at;
-    at += c;
   }
-  ids.resize(at);
-  each([&](uint32_t t, uint32_t gid) { ids[count[t]++] = gid; });
 }
 
 }  // namespace gsr
