@@ -24,6 +24,7 @@ std::vector<TuneChoice> tune_candidates() {
     for (uint32_t chunk : {256u, 128u, 64u}) {
       TuneChoice t;
       t.tile = 16;
+      t.raster.chosen = true;
       t.raster.chunk = chunk;
       t.raster.blocks_per_sm = bps;
       c.push_back(t);
@@ -32,6 +33,7 @@ std::vector<TuneChoice> tune_candidates() {
     for (uint32_t chunk : {64u, 32u}) {
       TuneChoice t;
       t.tile = 8;
+      t.raster.chosen = true;
       t.raster.chunk = chunk;
       t.raster.blocks_per_sm = bps;
       c.push_back(t);
@@ -73,6 +75,7 @@ bool tune_cache_lookup(const std::string &path, const std::string &key, TuneChoi
     if (!std::getline(ls, k, '\t')) continue;
     if (!(ls >> c.tile >> c.raster.chunk >> c.raster.blocks_per_sm >> c.ms)) continue;
     if (k == key && (c.tile == 8 || c.tile == 16) && raster_config_valid(c.tile, c.raster)) {
+      c.raster.chosen = true;
       out = c;  // the last entry for a key wins
       found = true;
     }

@@ -368,6 +368,7 @@ int32_t gsplat_context_set_raster_config(GsplatContext *ctx, uint32_t chunk, uin
     gsr::RasterConfig c;
     c.chunk = chunk;
     c.blocks_per_sm = blocks_per_sm;
+    c.chosen = true;
     ctx->renderer->set_raster_config(c);
     return ok();
   });
@@ -793,6 +794,7 @@ int32_t gsplat_batch_set_raster_config(GsplatBatch *batch, uint32_t chunk, uint3
     gsr::RasterConfig c;
     c.chunk = chunk;
     c.blocks_per_sm = blocks_per_sm;
+    c.chosen = true;
     batch->batch->set_raster_config(c);
     return ok();
   });

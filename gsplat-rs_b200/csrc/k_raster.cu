@@ -982,6 +982,11 @@ void launch_raster(const RasterArgs &a, uint32_t tile, uint32_t blend_mode,
 #undef GSR_FP32
 }
 
+RasterConfig raster_config_at(uint32_t tile, RasterConfig cfg) {
+  if (cfg.chosen && raster_config_valid(tile, cfg)) return cfg;
+  return {tile * tile, cfg.blocks_per_sm, false};
+}
+
 bool raster_config_valid(uint32_t tile, const RasterConfig &cfg) {
   const bool chunk_ok = tile == 16 ? (cfg.chunk == 64 || cfg.chunk == 128 || cfg.chunk == 256)
                                    : (cfg.chunk == 32 || cfg.chunk == 64);

@@ -142,19 +142,24 @@ struct RasterArgs {
   unsigned long long *end_ns;      // pinned: when the raster ends, if wanted
   float2 *debug_cov = nullptr;     // debug tap: (log2 alpha, coverage bound) per splat slot
 };
-// Raster launch shape: records staged per step (tile 16: 64/128/256; tile 8:
+// Raster launch shape of the FP32 mode: the chunk (tile 16: 64/128/256; tile 8:
 // 32/64) and persistent blocks per SM pulling tiles from a global queue
-// (0 = one block per tile). The FP32 mode honours both; UNORM8 parity mode
-// always runs one block per tile with full-tile chunks. No setting changes a
-// pixel.
+// (0 = one block per tile). A chunk below the full tile (256, 64) is the
+// records staged per step; the full tile leaves the step to the run's number of
+// tiles (launch_raster). UNORM8 parity mode takes neither: it runs one block per
+// tile with steps of its own. No setting changes a pixel.
 struct RasterConfig {
   uint32_t chunk = 256;
   uint32_t blocks_per_sm = 0;
+  bool chosen = false;  // set by a caller: kept over a change of tile size where it is valid
   bool operator==(const RasterConfig &o) const {
     return chunk == o.chunk && blocks_per_sm == o.blocks_per_sm;
   }
 };
 bool raster_config_valid(uint32_t tile, const RasterConfig &cfg);
+// The configuration after a change to tile size `tile`: a chunk that is not
+// valid there, or that no caller chose, becomes the full tile.
+RasterConfig raster_config_at(uint32_t tile, RasterConfig cfg);
 void launch_raster(const RasterArgs &a, uint32_t tile, uint32_t blend_mode,
                    const RasterConfig &cfg, uint32_t sm_count, cudaStream_t stream);
 

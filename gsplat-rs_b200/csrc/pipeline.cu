@@ -184,7 +184,7 @@ Pipeline::~Pipeline() {
 
 void Pipeline::set_tile(uint32_t tile) {
   tile_ = tile;
-  if (!raster_config_valid(tile_, raster_cfg_)) raster_cfg_.chunk = tile_ * tile_;
+  raster_cfg_ = raster_config_at(tile_, raster_cfg_);
 }
 
 void Pipeline::set_raster_config(const RasterConfig &c) {

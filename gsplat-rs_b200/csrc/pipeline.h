@@ -111,7 +111,7 @@ class Pipeline {
   Pipeline(int device, cudaStream_t stream);
   ~Pipeline();
 
-  // Tile size 8 or 16; the raster chunk follows to the nearest valid size.
+  // Tile size 8 or 16; the raster chunk follows (raster_config_at).
   void set_tile(uint32_t tile);
   uint32_t tile() const { return tile_; }
   void set_blend_mode(uint32_t mode) { blend_mode_ = mode; }

@@ -94,11 +94,15 @@ int32_t gsplat_context_set_debug_taps(GsplatContext *ctx, uint32_t enabled);
  * taps and pair capacity stay the same; disabled, every launch is issued
  * separately. Images are identical either way. */
 int32_t gsplat_context_set_cuda_graph(GsplatContext *ctx, uint32_t enabled);
-/* Raster launch shape of the FP32 mode: records staged per step (`chunk`:
- * 64, 128 or 256 at tile size 16; 32 or 64 at tile size 8) and persistent
- * blocks per SM that pull tiles from a global queue (0 = one block per tile,
- * at most 32). Changing the tile size resets an invalid chunk to the full
- * tile. Images do not depend on either setting. */
+/* Raster launch shape of the FP32 mode: `chunk` (64, 128 or 256 at tile size
+ * 16; 32 or 64 at tile size 8) and persistent blocks per SM that pull tiles
+ * from a global queue (0 = one block per tile, at most 32). A chunk below the
+ * full tile (256, 64) is the records staged per step. The full tile, the
+ * default, leaves the step to the number of tiles of the run: 256 records up to
+ * 7 tiles per SM and 128 above at tile size 16, 128 up to 16 tiles per SM and 64
+ * above at tile size 8; only it has the kernels for few tiles. Changing the
+ * tile size resets a chunk that is invalid there, or was never set, to the full
+ * tile. The UNORM8 mode takes neither setting. Images do not depend on them. */
 int32_t gsplat_context_set_raster_config(GsplatContext *ctx, uint32_t chunk, uint32_t blocks_per_sm);
 /* Depth-order refresh cadence. 0 (the default) sorts every frame, as the
  * reference's gsplat_context_render_frame does. interval >= 1 applies the

@@ -3,6 +3,7 @@
 // dynamic shared memory it asks for, the limit raised for that kernel on that
 // device (0: none), and the launch's priority attribute ("-": none).
 //   launch_probe preprocess|emit|sort|sort-high
+// "raster-tile" prints the chunk kept over changes of the tile size.
 // "work" prints pair capacities, the words of their sort's scratch and the bytes
 // a pair is counted with in place of launches.
 #include <cuda_runtime.h>
@@ -117,6 +118,18 @@ int main(int argc, char **argv) {
           b.passes = bits ? 1 : 4;
           b.wide_bits = bits;
           launch_sort(b, nullptr);
+        }
+    } else if (!std::strcmp(what, "raster-tile")) {
+      // chunk (0: never set) at a first tile size, then at the other, then back
+      for (uint32_t tile : {16u, 8u})
+        for (uint32_t chunk : {0u, 32u, 64u, 128u, 256u}) {
+          RasterConfig c = raster_config_at(tile, RasterConfig{});
+          if (chunk) c = {chunk, 3, true};
+          if (!raster_config_valid(tile, c)) continue;
+          const RasterConfig there = raster_config_at(24 - tile, c);
+          const RasterConfig back = raster_config_at(tile, there);
+          std::printf("raster-tile %u %u %u %u %u %u\n", tile, chunk, there.chunk, back.chunk,
+                      there.blocks_per_sm, back.blocks_per_sm);
         }
     } else if (!std::strcmp(what, "work")) {
       for (uint32_t capacity : {1u << 20, 3'000'001u, 1u << 28})

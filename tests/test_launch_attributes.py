@@ -9,7 +9,7 @@ import pytest
 import build as native
 from conftest import ROOT
 
-OBJECTS = ("k_preprocess.cu.o", "k_tiles.cu.o", "k_sort.cu.o")
+OBJECTS = ("k_preprocess.cu.o", "k_tiles.cu.o", "k_sort.cu.o", "k_raster.cu.o")
 
 
 @pytest.fixture(scope="module")
@@ -29,7 +29,7 @@ def probe(tmp_path_factory):
         return [(int(d), int(smem), int(limit), prio)
                 for d, smem, limit, prio in lines(what, "launch")]
 
-    run.values = lambda what: [tuple(map(int, row)) for row in lines(what, "work")]
+    run.values = lambda what: [tuple(map(int, row)) for row in lines(what, what)]
     return run
 
 
@@ -57,3 +57,13 @@ def test_admitted_pair_bytes_cover_the_workspace(probe):
     and values twice and the sort's scratch."""
     for capacity, words, counted in probe.values("work"):
         assert 16 * capacity + 4 * words <= counted * capacity + (1 << 16), (capacity, words)
+
+
+def test_raster_chunk_over_changes_of_the_tile_size(probe):
+    """A chunk that was never set is the full tile at either tile size; one that
+    was set stays where it is valid and becomes the full tile where it is not."""
+    rows = {(tile, chunk): rest for tile, chunk, *rest in probe.values("raster-tile")}
+    assert rows == {
+        (16, 0): [64, 256, 0, 0], (16, 64): [64, 64, 3, 3], (16, 128): [64, 256, 3, 3],
+        (16, 256): [64, 256, 3, 3], (8, 0): [256, 64, 0, 0], (8, 32): [256, 64, 3, 3],
+        (8, 64): [64, 64, 3, 3]}
