@@ -1,7 +1,10 @@
 // Autotuner of the batched launch shape: tile size (8 or 16), raster chunk
-// size (records staged per step) and persistent raster blocks per SM. Every
-// candidate renders the caller's views with the caller's batch; the fastest
-// by median device time wins and is applied to the batch. Results persist in
+// size and persistent raster blocks per SM. Every candidate renders the
+// caller's views with the caller's batch; the fastest by median device time
+// wins and is applied to the batch. Candidates that launch the same kernels for
+// these views (chunks 256 and 128 with many tiles, all of a tile size in the
+// UNORM8 mode) are timed once and the first of them stands for them: timed each,
+// the choice among them was noise, and was cached. Results persist in
 // a small text file keyed by GPU name, blend mode, the set of image sizes and
 // the scene-size class, so later processes reuse them without searching. No
 // candidate changes a pixel, only the time.

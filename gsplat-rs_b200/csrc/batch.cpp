@@ -292,6 +292,17 @@ void Batch::set_limits(const GroupLimits &l) {
   limits_ = l;
 }
 
+std::vector<GroupShape> Batch::group_shapes() {
+  std::vector<GroupShape> out;
+  for (const ViewGroup &g : groups_) {
+    uint32_t tiles = 0;
+    for (uint32_t v = g.first; v < g.first + g.count; ++v)
+      tiles += ((specs_[v].width + tile_ - 1) / tile_) * ((specs_[v].height + tile_ - 1) / tile_);
+    out.push_back({g.first, g.count, lane_->pipe().raster_shape_of(tiles)});
+  }
+  return out;
+}
+
 BatchResult Batch::render(const std::vector<BatchView> &in) {
   auto t0 = std::chrono::steady_clock::now();
   if (in.empty()) throw Error(Code::InvalidArgument, "no views to render");

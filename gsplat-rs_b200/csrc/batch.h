@@ -79,6 +79,15 @@ struct ViewGroup {
   uint64_t predicted_pairs;
 };
 
+// A launch group of a render: its views and what its raster launched.
+struct GroupShape {
+  uint32_t first, count;
+  RasterShape raster;
+  bool operator==(const GroupShape &o) const {
+    return first == o.first && count == o.count && raster == o.raster;
+  }
+};
+
 // Splits views, in order, into launch groups within `limits`.
 std::vector<ViewGroup> plan_groups(const std::vector<ViewSpec> &views,
                                    const std::vector<uint64_t> &predicted, uint32_t tile,
@@ -175,6 +184,7 @@ class Batch {
 
   // Renders every view; blocks until all images are in HBM.
   BatchResult render(const std::vector<BatchView> &views);
+  std::vector<GroupShape> group_shapes();  // of the last render
   uint32_t view_count() const { return (uint32_t)specs_.size(); }
   // Per-view results by the caller's view index.
   const ViewCounters &view_stats(uint32_t view) const;

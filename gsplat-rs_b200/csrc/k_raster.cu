@@ -930,27 +930,58 @@ __global__ void __launch_bounds__(kTile *kTile / kPx, kBlocks)
 
 }  // namespace
 
+// With few tiles the one with the longest list sets the time, and a warp of
+// it is bound by its own latencies: the registers that no further block
+// would use go to it (4 or 7 blocks a SM instead of 8, 8 of 8x8 tiles
+// instead of 16), its list is walked ahead, and the steps are longer (us, 8
+// blocks and a direct walk -> as here: 256 tiles of 27 k pairs 32.8 -> 28.7,
+// 190 tiles, 62 k splats 110.6 -> 84.0, 475 tiles, 2 M splats 71.7 -> 49.2;
+// 750 tiles of 100 k splats 59.4 -> 55.3 at 7 blocks). A chunk is the most a
+// step stages: with more tiles than blocks are resident half of 256 is
+// better, since a tile that fills up early has then gathered fewer records
+// it does not need and 8 blocks fit (1.70 M pairs at 1920x1080 116.9 ->
+// 112.6 us, 186 M at 3840x2160 500 -> 397). UNORM8: at most 4 tiles a SM (16
+// of 8x8 pixels), see raster_unorm8_kernel.
+RasterShape raster_shape(uint32_t total_tiles, uint32_t tile, uint32_t blend_mode,
+                         const RasterConfig &cfg, uint32_t sm_count) {
+  if (blend_mode == 1) {
+    const bool ahead = total_tiles <= (tile == 16 ? 4 : 16) * sm_count;
+    const uint32_t chunk = tile == 16   ? (ahead ? U8Smem<16, true>::kChunk : U8Smem<16, false>::kChunk)
+                           : ahead      ? U8Smem<8, true>::kChunk
+                                        : U8Smem<8, false>::kChunk;
+    return {tile, blend_mode, chunk, ahead, 0};
+  }
+  const uint32_t per_sm = (total_tiles + sm_count - 1) / sm_count;
+  uint32_t chunk = cfg.chunk, blocks = tile == 16 ? kManyBlocks<16> : kManyBlocks<8>;
+  if (tile == 16 && chunk == 256) {
+    if (per_sm > 7) chunk = 128;
+    else blocks = per_sm > 4 ? 7 : 4;
+  } else if (tile == 8 && chunk == 64 && per_sm <= 16) {
+    chunk = 128;
+    blocks = 8;
+  }
+  return {tile, blend_mode, chunk, blocks, cfg.blocks_per_sm};
+}
+
 void launch_raster(const RasterArgs &a, uint32_t tile, uint32_t blend_mode,
                    const RasterConfig &cfg, uint32_t sm_count, cudaStream_t stream) {
   if (a.total_tiles == 0) return;
+  const RasterShape s = raster_shape(a.total_tiles, tile, blend_mode, cfg, sm_count);
   if (blend_mode == 1) {
-    // At most 4 tiles a SM (16 of 8x8 pixels): see raster_unorm8_kernel.
-    const bool ahead = a.total_tiles <= (tile == 16 ? 4 : 16) * sm_count;
 #define GSR_U8(T, A) raster_unorm8_kernel<T, A><<<a.total_tiles, T * T, 0, stream>>>(a)
     if (tile == 16) {
-      if (ahead) GSR_U8(16, true);
+      if (s.blocks) GSR_U8(16, true);
       else GSR_U8(16, false);
     } else {
-      if (ahead) GSR_U8(8, true);
+      if (s.blocks) GSR_U8(8, true);
       else GSR_U8(8, false);
     }
 #undef GSR_U8
     return;
   }
-  const bool persistent = cfg.blocks_per_sm > 0;
+  const bool persistent = s.blocks_per_sm > 0;
   const uint32_t grid =
-      persistent ? std::min<uint32_t>(a.total_tiles, cfg.blocks_per_sm * sm_count) : a.total_tiles;
-  const uint32_t per_sm = (a.total_tiles + sm_count - 1) / sm_count;
+      persistent ? std::min<uint32_t>(a.total_tiles, s.blocks_per_sm * sm_count) : a.total_tiles;
 #define GSR_FP32(T, C, P, B)                                                     \
   do {                                                                           \
     if (persistent)                                                              \
@@ -958,25 +989,14 @@ void launch_raster(const RasterArgs &a, uint32_t tile, uint32_t blend_mode,
     else                                                                         \
       raster_fp32_kernel<T, C, P, B, false><<<grid, T * T / P, 0, stream>>>(a);  \
   } while (0)
-  // With few tiles the one with the longest list sets the time, and a warp of
-  // it is bound by its own latencies: the registers that no further block
-  // would use go to it (4 or 7 blocks a SM instead of 8, 8 of 8x8 tiles
-  // instead of 16), its list is walked ahead, and the steps are longer (us, 8
-  // blocks and a direct walk -> as here: 256 tiles of 27 k pairs 32.8 -> 28.7,
-  // 190 tiles, 62 k splats 110.6 -> 84.0, 475 tiles, 2 M splats 71.7 -> 49.2;
-  // 750 tiles of 100 k splats 59.4 -> 55.3 at 7 blocks). A chunk is the most a
-  // step stages: with more tiles than blocks are resident half of 256 is
-  // better, since a tile that fills up early has then gathered fewer records
-  // it does not need and 8 blocks fit (1.70 M pairs at 1920x1080 116.9 ->
-  // 112.6 us, 186 M at 3840x2160 500 -> 397).
   if (tile == 16) {
-    if (cfg.chunk == 64) GSR_FP32(16, 64, GSR_RASTER_PX, kManyBlocks<16>);
-    else if (cfg.chunk == 128 || per_sm > 7) GSR_FP32(16, 128, GSR_RASTER_PX, kManyBlocks<16>);
-    else if (per_sm > 4) GSR_FP32(16, 256, GSR_RASTER_PX, 7);
+    if (s.chunk == 64) GSR_FP32(16, 64, GSR_RASTER_PX, kManyBlocks<16>);
+    else if (s.chunk == 128) GSR_FP32(16, 128, GSR_RASTER_PX, kManyBlocks<16>);
+    else if (s.blocks == 7) GSR_FP32(16, 256, GSR_RASTER_PX, 7);
     else GSR_FP32(16, 256, GSR_RASTER_PX, 4);
   } else {
-    if (cfg.chunk == 32) GSR_FP32(8, 32, 1, kManyBlocks<8>);
-    else if (per_sm > 16) GSR_FP32(8, 64, 1, kManyBlocks<8>);
+    if (s.chunk == 32) GSR_FP32(8, 32, 1, kManyBlocks<8>);
+    else if (s.chunk == 64) GSR_FP32(8, 64, 1, kManyBlocks<8>);
     else GSR_FP32(8, 128, 1, 8);
   }
 #undef GSR_FP32

@@ -146,7 +146,7 @@ struct RasterArgs {
 // 32/64) and persistent blocks per SM pulling tiles from a global queue
 // (0 = one block per tile). A chunk below the full tile (256, 64) is the
 // records staged per step; the full tile leaves the step to the run's number of
-// tiles (launch_raster). UNORM8 parity mode takes neither: it runs one block per
+// tiles (raster_shape). UNORM8 parity mode takes neither: it runs one block per
 // tile with steps of its own. No setting changes a pixel.
 struct RasterConfig {
   uint32_t chunk = 256;
@@ -160,6 +160,20 @@ bool raster_config_valid(uint32_t tile, const RasterConfig &cfg);
 // The configuration after a change to tile size `tile`: a chunk that is not
 // valid there, or that no caller chose, becomes the full tile.
 RasterConfig raster_config_at(uint32_t tile, RasterConfig cfg);
+// What a run of `total_tiles` tiles launches for a configuration: runs of equal
+// shapes launch the same kernel on the same grid.
+struct RasterShape {
+  uint32_t tile, blend_mode;
+  uint32_t chunk;          // records per step
+  uint32_t blocks;         // blocks an SM the kernel is compiled for (FP32), or 1: few tiles (UNORM8)
+  uint32_t blocks_per_sm;  // persistent blocks, 0: one block per tile
+  bool operator==(const RasterShape &o) const {
+    return tile == o.tile && blend_mode == o.blend_mode && chunk == o.chunk &&
+           blocks == o.blocks && blocks_per_sm == o.blocks_per_sm;
+  }
+};
+RasterShape raster_shape(uint32_t total_tiles, uint32_t tile, uint32_t blend_mode,
+                         const RasterConfig &cfg, uint32_t sm_count);
 void launch_raster(const RasterArgs &a, uint32_t tile, uint32_t blend_mode,
                    const RasterConfig &cfg, uint32_t sm_count, cudaStream_t stream);
 

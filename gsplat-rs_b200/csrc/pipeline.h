@@ -129,6 +129,9 @@ class Pipeline {
   // Throws InvalidArgument unless valid for the current tile size.
   void set_raster_config(const RasterConfig &c);
   const RasterConfig &raster_config() const { return raster_cfg_; }
+  RasterShape raster_shape_of(uint32_t total_tiles) const {
+    return raster_shape(total_tiles, tile_, blend_mode_, raster_cfg_, sm_count_);
+  }
 
   // Renders `count` views into `images` (device, RGBA8 words) at the given
   // pixel offsets and waits. Grows the pair buffers and re-runs on overflow.

@@ -302,7 +302,7 @@ typedef struct GsplatTuneResult {
   uint32_t tile_size;      /* chosen launch shape, now set on the batch */
   uint32_t chunk;
   uint32_t blocks_per_sm;
-  uint32_t candidates;     /* shapes timed (0 when taken from the cache) */
+  uint32_t candidates;     /* shapes compared (0 when taken from the cache) */
   float best_ms;           /* median device time of the views with it */
   float default_ms;        /* the same with tile 16, chunk 256, one block per tile */
   uint32_t from_cache;
@@ -313,7 +313,8 @@ typedef struct GsplatTuneResult {
  * candidate (tile 16 with chunks 256/128/64, tile 8 with chunks 64/32, each
  * with one block per tile or 2/4 resp. 8/16 persistent blocks per SM), keeps
  * the fastest by median device time over `reps` renders and sets it on the
- * batch. With a `cache_path`, results are kept in that text file keyed by GPU
+ * batch. Candidates that launch the same kernels for these views are timed
+ * once; the first of them stands for them. With a `cache_path`, results are kept in that text file keyed by GPU
  * name, blend mode, image sizes and scene-size class, and a later call with
  * the same key takes the stored shape without rendering. Images are the same
  * under every candidate. */

@@ -3,7 +3,9 @@
 // dynamic shared memory it asks for, the limit raised for that kernel on that
 // device (0: none), and the launch's priority attribute ("-": none).
 //   launch_probe preprocess|emit|sort|sort-high
-// "raster-tile" prints the chunk kept over changes of the tile size.
+// "raster" prints the shape raster_shape names for every configuration and
+// number of tiles, and the kernel (as a number) and grid launch_raster launches
+// for it; "raster-tile" the chunk kept over changes of the tile size.
 // "work" prints pair capacities, the words of their sort's scratch and the bytes
 // a pair is counted with in place of launches.
 #include <cuda_runtime.h>
@@ -20,7 +22,13 @@ namespace {
 int device = 0;
 std::map<std::pair<int, const void *>, int> limits;
 
-void note(const void *func, size_t smem, const char *priority) {
+std::map<const void *, int> kernels;
+int last_kernel = -1;
+unsigned last_grid = 0;
+
+void note(const void *func, size_t smem, const char *priority, dim3 grid) {
+  last_kernel = kernels.emplace(func, (int)kernels.size()).first->second;
+  last_grid = grid.x;
   auto it = limits.find({device, func});
   std::printf("launch %d %zu %d %s\n", device, smem, it == limits.end() ? 0 : it->second, priority);
 }
@@ -52,8 +60,8 @@ cudaError_t __cudaPopCallConfiguration(dim3 *grid, dim3 *block, size_t *smem, vo
   *(cudaStream_t *)stream = config.stream;
   return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void *func, dim3, dim3, void **, size_t smem, cudaStream_t) {
-  note(func, smem, "-");
+cudaError_t cudaLaunchKernel(const void *func, dim3 grid, dim3, void **, size_t smem, cudaStream_t) {
+  note(func, smem, "-", grid);
   return cudaSuccess;
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *func, void **) {
@@ -61,7 +69,7 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *func, v
   for (unsigned k = 0; k < c->numAttrs; ++k)
     if (c->attrs[k].id == cudaLaunchAttributePriority)
       std::snprintf(priority, sizeof priority, "%d", c->attrs[k].val.priority);
-  note(func, c->dynamicSmemBytes, priority);
+  note(func, c->dynamicSmemBytes, priority, c->gridDim);
   return cudaSuccess;
 }
 cudaError_t cudaFuncSetAttribute(const void *func, cudaFuncAttribute attr, int value) {
@@ -119,6 +127,22 @@ int main(int argc, char **argv) {
           b.wide_bits = bits;
           launch_sort(b, nullptr);
         }
+    } else if (!std::strcmp(what, "raster")) {
+      for (uint32_t tiles : {1u, 592u, 593u, 1036u, 1037u, 2368u, 2369u, 8160u})
+        for (uint32_t mode : {0u, 1u})
+          for (uint32_t tile : {8u, 16u})
+            for (uint32_t chunk : {32u, 64u, 128u, 256u})
+              for (uint32_t bps : {0u, 2u}) {
+                const RasterConfig cfg{chunk, bps, true};
+                if (!raster_config_valid(tile, cfg)) continue;
+                const RasterShape s = raster_shape(tiles, tile, mode, cfg, 148);
+                RasterArgs a{};
+                a.total_tiles = tiles;
+                launch_raster(a, tile, mode, cfg, 148, nullptr);
+                std::printf("raster %u %u %u %u %u %u %u %u %u %d %u\n", tiles, mode, tile, chunk,
+                            bps, s.chunk, s.blocks, s.blocks_per_sm, s.tile + 100 * s.blend_mode,
+                            last_kernel, last_grid);
+              }
     } else if (!std::strcmp(what, "raster-tile")) {
       // chunk (0: never set) at a first tile size, then at the other, then back
       for (uint32_t tile : {16u, 8u})

@@ -59,6 +59,22 @@ def test_admitted_pair_bytes_cover_the_workspace(probe):
         assert 16 * capacity + 4 * words <= counted * capacity + (1 << 16), (capacity, words)
 
 
+def test_raster_shapes_are_what_is_launched(probe):
+    """The autotuner compares candidates by the shape raster_shape names: equal
+    shapes are one kernel on one grid, different ones are not. A chunk below
+    the full tile is the step; the full tile's follows the number of tiles."""
+    rows = set(probe.values("raster"))
+    by_tiles = {}
+    for tiles, mode, tile, chunk, bps, *shape, kernel, grid in rows:
+        by_tiles.setdefault(tiles, set()).add((tuple(shape), kernel, grid))
+        full = {16: 256 if tiles <= 7 * 148 else 128, 8: 128 if tiles <= 16 * 148 else 64}[tile]
+        if mode == 0:
+            assert shape[0] == (chunk if chunk < tile * tile else full)
+        assert shape[2] == (0 if mode else bps)
+    for pairs in by_tiles.values():
+        assert len({s for s, *_ in pairs}) == len({k[1:] for k in pairs}) == len(pairs)
+
+
 def test_raster_chunk_over_changes_of_the_tile_size(probe):
     """A chunk that was never set is the full tile at either tile size; one that
     was set stays where it is valid and becomes the full tile where it is not."""
