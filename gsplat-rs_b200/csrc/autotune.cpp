@@ -9,6 +9,7 @@
 #include <map>
 #include <set>
 #include <sstream>
+#include <utility>
 
 #include "cuda_check.h"
 
@@ -136,8 +137,16 @@ TuneResult autotune(Batch &batch, const std::vector<BatchView> &views, const std
     for (TuneChoice c : tune_candidates()) {
       batch.set_tile(c.tile);
       batch.set_raster_config(c.raster);
-      batch.render(views);  // warm-up: buffers, pair predictions, graph
+      // Warm-up until a launch of groups repeats: the first candidate's first
+      // render plans them without pair predictions, a layout's first render
+      // launches directly and its second captures the graph the timed ones run.
+      batch.render(views);
       launched.push_back(batch.group_shapes());
+      for (int k = 0; k < 4; ++k) {
+        batch.render(views);
+        const std::vector<GroupShape> before = std::exchange(launched.back(), batch.group_shapes());
+        if (launched.back() == before) break;
+      }
       // one that launches what an earlier one did has its time
       const size_t same = std::find(launched.begin(), launched.end(), launched.back()) - launched.begin();
       if (same < r.tried.size()) {
@@ -149,7 +158,6 @@ TuneResult autotune(Batch &batch, const std::vector<BatchView> &views, const std
       for (uint32_t k = 0; k < reps; ++k) ms.push_back(batch.render(views).device_ms);
       std::sort(ms.begin(), ms.end());
       c.ms = ms[ms.size() / 2];
-      launched.back() = batch.group_shapes();  // the first render had no pair predictions
       r.tried.push_back(c);
       if (r.tried.size() == 1) r.default_ms = c.ms;
     }

@@ -30,3 +30,19 @@ def test_equal_candidates_are_one(blend):
             assert r.chunk != 128
         b.render(views)
         assert np.array_equal(b.readback_rgba8(0), before)
+
+
+def test_candidates_are_timed_on_the_graph_they_run():
+    """The default shape's time is that of its repeated render, one graph
+    launch: the renders that plan without predictions and that capture the
+    graph (host milliseconds between the launches of well under one) are not
+    timed. The margin is for a busy host and the clocks."""
+    scene, cam, _, _ = gsplat_scenes.config1(seed=6)
+    views = [(0, cam, 400 + 16 * k, 300) for k in range(12)]
+    with ffi.Batch() as b:
+        b.add_scene(scene)
+        r = b.autotune(views, None, reps=1)
+        b.set_tile_size(16)
+        b.set_raster_config(256, 0)
+        steady = sorted(b.render(views).device_ms for _ in range(9))[4]
+        assert r.default_ms < 2.0 * steady, (r.default_ms, steady)
