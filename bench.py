@@ -222,6 +222,48 @@ def algorithmic_bytes(phase, counts, n, planes, width, height, passes):
     return 0
 
 
+def phase_rows(phase_ms, bytes_of, peaks):
+    """Rows of a phase table: device ms, algorithmic bytes and the GB/s they
+    make, with a fraction of each of `peaks` (name -> GB/s). The depth sort runs
+    beside the vertex stage, so its own ms is what it takes beyond that (near 0
+    where the vertex stage is the longer) and says nothing about its rate: the
+    two have one rate together, in the row preprocess_depth_sort."""
+    beside = ("preprocess", "depth_sort")
+    rows = {k: {"ms": ms, "bytes": bytes_of(k)} for k, ms in phase_ms.items()}
+    if all(k in rows for k in beside):
+        rows["preprocess_depth_sort"] = {f: sum(rows[k][f] for k in beside)
+                                         for f in ("ms", "bytes")}
+    for k, row in rows.items():
+        if k in beside:
+            continue
+        row["gbs"] = row["bytes"] / (row["ms"] * 1e-3) / 1e9 if row["ms"] > 0 else None
+        for name, peak in peaks.items():
+            row["frac_" + name] = row["gbs"] / peak if row["gbs"] else None
+    return rows
+
+
+def batched_phase_rows(phase_ms, specs, stats, scenes, planes, hbm):
+    """Phase table of a batch: the views' bytes, the scenes read once per view
+    set, and the passes of each launch group's bins."""
+    group_bins = {}
+    for st, (_, _, w, h) in zip(stats, specs):
+        group_bins[st.group] = group_bins.get(st.group, 0) + view_bins(w, h)
+    group_passes = {g: bin_passes(bins) for g, bins in group_bins.items()}
+
+    def bytes_of(phase):
+        if phase == "preprocess":
+            return batched_preprocess_bytes(specs, stats, scenes, planes)
+        total = 0
+        for st, (sid, _, w, h) in zip(stats, specs):
+            c = types.SimpleNamespace(visible=st.visible_count, drawn=st.drawn_count,
+                                      tile_keys=st.tile_pairs)
+            total += algorithmic_bytes(phase, c, scenes[sid]["positions"].shape[0], planes, w, h,
+                                       group_passes[st.group])
+        return total
+
+    return phase_rows(phase_ms, bytes_of, {"measured": hbm})
+
+
 def batched_preprocess_bytes(specs, stats, scenes, planes, set_views=16):
     """Preprocess bytes of a batch at minimum: a view set (up to `set_views`
     consecutive views of one scene in a launch group, in render order: views
@@ -463,27 +505,8 @@ def measure_batched(ffi, torch, steps, warmup, cameras_per_scene=64):
     phase_ms = b.phase_times()
     b.set_phase_timing(False)
     stats = [b.view_stats(k) for k in range(len(specs))]
-    group_bins = {}
-    for k, (sid, _, w, h) in enumerate(specs):
-        g = stats[k].group
-        group_bins[g] = group_bins.get(g, 0) + view_bins(w, h)
-    group_passes = {g: bin_passes(bins) for g, bins in group_bins.items()}
     hbm = hbm_peak_gbs()
-    phases = {}
-    for k, ms in phase_ms.items():
-        if k == "preprocess":
-            nbytes = batched_preprocess_bytes(specs, stats, scenes, 12)
-        else:
-            nbytes = 0
-            for v, (sid, _, w, h) in enumerate(specs):
-                st = stats[v]
-                c = types.SimpleNamespace(visible=st.visible_count, drawn=st.drawn_count,
-                                          tile_keys=st.tile_pairs)
-                nbytes += algorithmic_bytes(k, c, scenes[sid]["positions"].shape[0], 12, w, h,
-                                            group_passes[st.group])
-        gbs = nbytes / (ms * 1e-3) / 1e9 if ms > 0 else None
-        phases[k] = {"ms": ms, "bytes": nbytes, "gbs": gbs,
-                     "frac_measured": gbs / hbm[0] if gbs else None}
+    phases = batched_phase_rows(phase_ms, specs, stats, scenes, 12, hbm[0])
     per_scene = []
     for sid in range(len(scenes)):
         sub = ffi.Batch.make_views([v for v in specs if v[0] == sid])
@@ -853,8 +876,10 @@ def measure_packed(ffi, torch, frames=60):
     d = np.abs(images["planes"] - images["packed"])[..., :3] / 255.0
     out["image_mean_abs_diff"] = float(d.mean())
     out["image_frac_over_3"] = float((d > 3.0 / 255.0).any(axis=-1).mean())
-    out["preprocess_speedup"] = (out["planes"]["phases_ms"]["preprocess"] /
-                                 out["packed"]["phases_ms"]["preprocess"])
+    # the vertex stage and the depth sort beside it
+    both = {f: sum(out[f]["phases_ms"][k] for k in ("preprocess", "depth_sort"))
+            for f in ("planes", "packed")}
+    out["preprocess_speedup"] = both["planes"] / both["packed"]
     return out
 
 
@@ -907,13 +932,9 @@ def measure_config3(ffi, torch, frames=20):
                 for k, v in ctx.phase_times().items():
                     acc.setdefault(k, []).append(v)
             ph = {k: float(np.median(v)) for k, v in acc.items()}
-            phases = {}
-            for k, ms in ph.items():
-                b = algorithmic_bytes(k, counts, n, 12, w, h, passes)
-                gbs = b / (ms * 1e-3) / 1e9 if ms > 0 else None
-                phases[k] = {"ms": ms, "bytes": b, "gbs": gbs,
-                             "frac_measured": gbs / hbm if gbs else None,
-                             "frac_nominal": gbs / NOMINAL_HBM_GBS if gbs else None}
+            phases = phase_rows(
+                ph, lambda k: algorithmic_bytes(k, counts, n, 12, w, h, passes),
+                {"measured": hbm, "nominal": NOMINAL_HBM_GBS})
             ps = ["preprocess", "depth_sort", "emit", "tile_sort"]
             ps_bytes = sum(phases[k]["bytes"] for k in ps)
             ps_ms = sum(phases[k]["ms"] for k in ps)
@@ -1107,10 +1128,9 @@ def run_cuda(args, world, rank, local):
             roofline["fp32_tflops"] = NCU_RASTER["thread_flop"] / raster_s / 1e12
             roofline["fp32_frac"] = roofline["fp32_tflops"] / fp32_peak
             roofline["counters_source"] = NCU_RASTER["source"]
-    phase_rooflines = {}
-    for k, ms in phases.items():
-        b = algorithmic_bytes(k, counts, scene["positions"].shape[0], planes, w, h, passes)
-        phase_rooflines[k] = {"ms": ms, "bytes": b, "gbs": b / (ms * 1e-3) / 1e9 if ms > 0 else None}
+    phase_rooflines = phase_rows(
+        phases, lambda k: algorithmic_bytes(k, counts, scene["positions"].shape[0], planes, w, h,
+                                            passes), {})
 
     # scratch zeroing; keys; depth sort: plan + 4 passes (histograms from the
     # keys); vertex stage; emit; bin sort: plan + passes (histograms from the
