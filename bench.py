@@ -204,7 +204,9 @@ def bin_passes(bins):
 def algorithmic_bytes(phase, counts, n, planes, width, height, passes):
     """Bytes each phase must move at minimum (reads + writes), per frame. The
     sorted pairs are (4x4-tile bin, splat) pairs, at least a sixteenth of the
-    tile pairs."""
+    tile pairs. The raster reads every drawn splat's record once and writes the
+    image: what it gathers per tile stays in L2, and less of it the sooner
+    pixels are opaque."""
     v, d, k = counts.visible, counts.drawn, counts.tile_keys
     b = k // 16
     if phase == "preprocess":
@@ -218,7 +220,7 @@ def algorithmic_bytes(phase, counts, n, planes, width, height, passes):
     if phase == "ranges":
         return b * 6
     if phase == "raster":
-        return k * 52 + width * height * 4
+        return d * 48 + width * height * 4
     return 0
 
 

@@ -32,6 +32,14 @@ def test_sort_beside_the_vertex_stage_has_no_rate_of_its_own():
     assert abs(rows["raster"]["gbs"] - 12.0) < 1e-9
 
 
+def test_raster_bytes_do_not_grow_with_the_tiles_a_splat_covers():
+    """A frame whose splats cover many tiles is opaque early: pairs are no
+    bound on what the raster reads, drawn records and the image are."""
+    few, many = (types.SimpleNamespace(visible=100, drawn=90, tile_keys=k) for k in (200, 10**9))
+    assert bench.algorithmic_bytes("raster", few, 120, 12, 64, 32, 1) == \
+        bench.algorithmic_bytes("raster", many, 120, 12, 64, 32, 1) == 90 * 48 + 64 * 32 * 4
+
+
 def test_batched_rows_sum_the_views():
     """Two groups: 1,200 bins (two passes) and 4 (one)."""
     specs = [(0, None, 1920, 2560), (0, None, 100, 100)]
@@ -41,4 +49,5 @@ def test_batched_rows_sum_the_views():
     rows = bench.batched_phase_rows({k: 1.0 for k in PHASES}, specs, stats, scenes, 12, 6000.0)
     assert rows["tile_sort"]["bytes"] == (2 + 1) * 100 * 16
     assert rows["preprocess"]["bytes"] == bench.batched_preprocess_bytes(specs, stats, scenes, 12)
+    assert rows["raster"]["bytes"] == 2 * 40 * 48 + 4 * (1920 * 2560 + 100 * 100)
     assert abs(rows["raster"]["frac_measured"] - rows["raster"]["bytes"] / 6e9) < 1e-12
