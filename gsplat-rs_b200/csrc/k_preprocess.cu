@@ -688,9 +688,14 @@ __global__ void __launch_bounds__(kK1Threads, GSR_K1_MIN_BLOCKS)
 // A frame's depth sort has about a block an SM (2,048 keys each), and each of
 // its passes waits for room beside the vertex stage, whose three blocks take
 // an SM's registers. Up to kTwoBlockTiles blocks the vertex stage asks for so
-// much shared memory that two fit and a sort block beside them (279k splats:
-// both together 73 -> 69 us); longer ones take all three (3M: 318 us against
-// 326, 1.0 M packed 146 against 151).
+// much shared memory that two fit and a sort block beside them; longer ones
+// take all three. Keys, sort and vertex stage together, three blocks against
+// two, us: SH3 279k splats (1,091 blocks) 68 / 66, 405k 80 / 77, 600k 94 / 90,
+// 800k 105 / 105, 1.0 M 123 / 130; packed 279k 61 / 62, 405k 76 / 74, 600k
+// 94 / 92, 800k 110 / 117; SH0, whose vertex stage is short, 279k 55 / 58, 405k
+// 67 / 70, 600k 79 / 83. So two blocks win by 2 to 4 us up to 2,000 to 2,500
+// blocks where the vertex stage is long and lose as much where it is short; the
+// line lies where the one is sure and the other small.
 constexpr size_t kTwoBlockSmem = 78'000;
 constexpr uint32_t kTwoBlockTiles = 1600;
 

@@ -324,8 +324,8 @@ __device__ __forceinline__ void pass_tile(const SortPlan *__restrict__ plan, uin
 // kMinBlocks: resident blocks per SM the register allocation must allow.
 // Sorts that leave L2 (tens of millions of keys and more) are latency bound
 // on their memory traffic and gain from a fourth resident block, though it
-// costs spills (64 registers); L2-resident sorts (a 1080p frame's 1.9 M tile
-// pairs) are faster with three.
+// costs spills (64 registers); L2-resident sorts (1.9 M pairs) are faster with
+// three.
 template <int kIpt, int kMinBlocks = (kIpt > 8 ? GSR_SORT_MIN_BLOCKS_LARGE : GSR_SORT_MIN_BLOCKS)>
 __global__ void __launch_bounds__(kThreads, kMinBlocks)
     pass_kernel(const SortPlan *__restrict__ plan, uint32_t pass, uint32_t shift, uint32_t *k0,
@@ -353,12 +353,12 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
 // ---- one wide pass ---------------------------------------------------------
 // A sort of 9 or 10 key bits (a bin sort of 257 to 1,024 bins) as one pass of
 // 512 or 1,024 digits, kDpt = 2 or 4 consecutive ones a thread, in place of two
-// passes of 256: 510 bins, 514k pairs 32.8 -> 24.6 us, 1,024 bins, 1.1 M pairs
-// 39.4 -> 36.9. Wider than that, or for sorts of more bits, 8-bit passes win: a
-// pass over 1.0 M keys takes 18 us with 256 digits, 22 with 512 and 30 with
-// 1,024, and 20.6 M pairs in 2,040 bins 334 us in one pass of 11 bits against
-// 297 in two. The 256-digit pass stays a kernel of its own: as this one's
-// kDpt = 1 form it ran 5% slower.
+// passes of 256 (plan and passes: 510 bins, 0.5 M pairs 26.2 -> 17.7 us; 1,024
+// bins, 279k and 600k splats at 2048x2048 29.0 -> 23.3 and 44.4 -> 36.4). Wider
+// than that, or for sorts of more bits, 8-bit passes win: a pass over 1.0 M keys
+// takes 18 us with 256 digits, 22 with 512 and 30 with 1,024, and 20.6 M pairs in
+// 2,040 bins 334 us in one pass of 11 bits against 297 in two. The 256-digit pass
+// stays a kernel of its own: as this one's kDpt = 1 form it ran 5% slower.
 constexpr int kWideIpt = 8;
 
 template <int kBits>

@@ -33,10 +33,16 @@ namespace {
 constexpr int kEmitThreads = 256;
 constexpr int kEmitWarps = kEmitThreads / 32;
 // Sorted ids per thread: 2 below kEmitLargeIds ids, 4 from there on, where
-// blocks of 1,024 ids still fill the GPU (4 resident per SM): fewer blocks,
-// each with its barriers, look-back and view table (1.0 M ids of 64 thumbnail
-// views 81 -> 71 us, 21 M ids of a mixed batch 1,852 -> 1,457 us); a 279k-id
-// frame takes 43 us instead of 33 with 4.
+// blocks of 1,024 ids fill the GPU (4 resident per SM): fewer blocks, each with
+// its barriers, look-back and view table (1.0 M ids of 64 thumbnail views 81 ->
+// 71 us, 21 M ids of a mixed batch 1,852 -> 1,457 us). A frame's emission with
+// 2 against 4, us: 279k ids 1280x720 25 / 29, 1920x1080 26 / 33; 350k 38 / 32
+// and 41 / 37; 420k 41 / 34 and 43 / 38; 500k 42 / 39 and 44 / 46; 560k 45 / 40
+// and 47 / 46; 650k 59 / 58 and 61 / 65; 900k 69 / 68 and 71 / 79; 1.1 M 85 / 73
+// and 90 / 84. The steps are the waves of resident blocks, 303k ids with 2 and
+// 606k with 4: up to 303k and, at 1920x1080, between 606k and 1.0 M 2 is faster,
+// from 303k to about 500k and beyond 1.1 M 4 is. The line was set by the ends
+// (279k and 1.0 M).
 constexpr uint64_t kEmitLargeIds = 600'000;
 // Units whose spans each warp keeps between its two walks (16 bytes each);
 // units past them are computed again in the second walk.

@@ -291,8 +291,9 @@ int32_t gsplat_batch_add_scene_packed(GsplatBatch *batch, const GsplatSceneDesc 
 int32_t gsplat_batch_set_tile_size(GsplatBatch *batch, uint32_t tile);       /* 8 or 16 */
 int32_t gsplat_batch_set_blend_mode(GsplatBatch *batch, uint32_t mode);      /* GsplatBlendMode */
 /* Launch-group limits: views (1..1024), predicted tile pairs, splats and
- * image tiles per group (0 keeps the current value). Up to 65,536 tiles a
- * group's tile sort takes two passes, above that three. */
+ * image tiles per group (0 keeps the current value). A group also holds at
+ * most 2^18 bins of 4x4 tiles over its views; its sort takes one pass up to
+ * 1,024 bins, two up to 65,536, three above. */
 int32_t gsplat_batch_set_limits(GsplatBatch *batch, uint32_t max_views, uint64_t max_pairs,
                                 uint64_t max_splats, uint64_t max_tiles);
 /* As gsplat_context_set_raster_config. */
