@@ -12,8 +12,8 @@
 // Why bins: a pair costs its write, one read and one write per sort pass and
 // the range build, whatever it covers. At 1920x1080 with 279k splats 1.70 M
 // (tile, splat) pairs become 0.51 M (bin, splat) pairs, at 3840x2160 with 3M
-// splats 186 M become 20.6 M: emission, tile sort and range build took 93 and
-// 3,730 us with tile pairs and take 76 and 805 us with bins. 4x4 because
+// splats 186 M become 20.6 M: emission, sort and range build took 93 and 3,730
+// us with tile pairs and take 48 and about 800 us with bins. 4x4 because
 // larger bins need longer codes and smaller ones leave more pairs; the 14 bits
 // leave 18 bits of bin id: the largest single view (16384x16384 at tile
 // size 8) has exactly 2^18 bins.
